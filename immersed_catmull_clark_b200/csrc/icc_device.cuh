@@ -41,6 +41,48 @@ struct Geom {
     int nbricks;
 };
 
+// Exact division of 0 <= n < 2^31 by a divisor fixed on the host: n / d = (n m) >> (31 + s) with
+// s = ceil(log2 d) and m = ceil(2^(31+s) / d).
+struct FastDiv {
+    unsigned m = 0x80000000u, s = 0;
+};
+inline FastDiv fast_div(unsigned d) {
+    FastDiv f;
+    while ((1ull << f.s) < d) ++f.s;
+    f.m = unsigned(((1ull << (31 + f.s)) + d - 1) / d);
+    return f;
+}
+__device__ __forceinline__ int operator/(int n, const FastDiv &f) {
+    return int(((unsigned long long)(unsigned)n * f.m) >> 31 >> f.s);
+}
+
+// A cut of the element grid into tiles of tx x ty x tz elements (the bricks of the dense paths are
+// one); a tile's partial sums cover its (tx + 2)(ty + 2)(tz + 2) control points, x fastest.  Tiles
+// are at least 2 long in a direction that has more than one, so a control point lies in <= 8.
+struct Tiles {
+    int tx, ty, tz, ltx;        // ltx = log2(tx)
+    int ntx, nty, ntz, n;
+    int vol;                    // partial sums of a tile, three components
+    FastDiv dx, dy, dz;         // division by tx, ty, tz
+    FastDiv dcx, dcy;           // division by the control points of a row and of a column
+};
+
+inline Tiles make_tiles(int nx, int ny, int nz, int tx, int ty, int tz) {
+    Tiles t;
+    t.tx = tx; t.ty = ty; t.tz = tz;
+    t.ltx = 0;
+    while ((1 << t.ltx) < tx) ++t.ltx;
+    t.ntx = (nx + tx - 1) / tx; t.nty = (ny + ty - 1) / ty; t.ntz = (nz + tz - 1) / tz;
+    t.n = t.ntx * t.nty * t.ntz;
+    t.vol = 3 * (tx + 2) * (ty + 2) * (tz + 2);
+    t.dx = fast_div((unsigned)tx); t.dy = fast_div((unsigned)ty); t.dz = fast_div((unsigned)tz);
+    t.dcx = fast_div((unsigned)nx + 2u); t.dcy = fast_div((unsigned)ny + 2u);
+    return t;
+}
+
+// The bricks of the dense paths as a tile cut (their partial sums are laid out the same way).
+inline Tiles brick_tiles(const Geom &g) { return make_tiles(g.nx, g.ny, g.nz, kBX, kBY, kBZ); }
+
 struct PcgState {
     double rz_old, p_ap, alpha, beta, norm_b, rel_res, tol;
     double rz_prev;        // r'z used by the last alpha (the beta of a residual replacement needs it)
@@ -82,6 +124,18 @@ __device__ __forceinline__ int edge_slot(const Edge &E, int d, int i) {
     return -1;
 }
 
+// Element matrices in Legendre modes (icc_modal.cuh), when a handle's matrices have that form: the
+// entries, the end factors per direction and the uniform element matrix (81 x 81) they stand for.
+struct ModalHost {
+    bool ok = false;
+    double diag[3][27], off[3][2][4][3], a[3], b[3];
+    std::vector<double> kunif;
+};
+struct ModalTile {
+    int nt = 0;   // columns (threads) of a tile
+    Tiles t{};
+};
+
 struct MixedState;  // tensor-core path (icc_mixed.cu)
 struct StateScratch;  // warm-started state solve and element energies (icc_topopt.cu)
 
@@ -97,7 +151,11 @@ struct Op {
     double *d_scale = nullptr, *d_kfrag = nullptr, *d_kdiag = nullptr;
     int *d_type_id = nullptr, *d_tile_start = nullptr, *d_tile_type = nullptr;
     uint8_t *d_tile_elem = nullptr, *d_mask = nullptr;
-    double *d_patch = nullptr;              // brick patch partial sums [nbricks][3][kPVol]
+    // FP64 apply: in Legendre modes on its own tiles when the matrices allow, else dense on bricks
+    ModalHost modal;
+    ModalTile mtile;                        // modal.ok: the FP64 tile
+    Tiles tiles{};                          // the cut the partial sums in d_patch belong to
+    double *d_patch = nullptr;              // tile partial sums [tiles.n][tiles.vol]
     // extra sparse term (icc_op_set_extra_triplets): y = mask rule of (K + S)(m .* x)
     int *d_sp_ptr = nullptr, *d_sp_idx = nullptr;
     double *d_sp_val = nullptr, *d_sp_diag = nullptr;
@@ -133,10 +191,12 @@ struct Op {
     ~Op();
     int init(const Space &s, const double *ke_types, int nt, const int32_t *type_id, const double *scale,
              const uint8_t *free_mask, int mode);
+    int init_dense();
     int set_scale(const double *scale);
     int set_scale_dev(const double *scale_dev);   // device array, stream-ordered
     int set_mask(const uint8_t *free_mask, int mode);
     int set_extra(int64_t count, const int64_t *rows, const int64_t *cols, const double *vals);
+    cudaError_t enqueue_contract(cudaStream_t s, const double *x, const PcgState *st);
     void enqueue_apply(const double *x, double *y, double *partials, const PcgState *st);
     void enqueue_apply_on(cudaStream_t s, const double *x, double *y);   // y = A x on stream s
     void enqueue_diagonal(double *d, cudaStream_t s);                     // the diagonal on stream s
@@ -149,6 +209,11 @@ struct Op {
 };
 
 int cuda_fail(cudaError_t e, const char *where);
+
+// operator in Legendre modes (icc_modal.cu)
+bool modal_setup(const Op &op, ModalHost &m);
+template <class T>
+ModalTile modal_tile(const Geom &g, int num_sms);
 
 // tensor-core mixed-precision path (icc_mixed.cu)
 void mixed_release(Op &op);

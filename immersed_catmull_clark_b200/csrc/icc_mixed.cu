@@ -1510,7 +1510,7 @@ static int enqueue_apply_tc(Op &op, const float *x, float *y) {
     ICC_CUDA(cudaMemcpyAsync(ms.d_inst, &I, sizeof(TcInst), cudaMemcpyHostToDevice, op.stream), "instance table");
     ICC_CUDA(launch_apply_tc(op.stream, ms.d_inst, 1, op.g.nbricks, ms.d_desc, ms.d_bmat, ms.d_err, op.num_sms),
              "tc apply launch");
-    gather_kernel<float><<<op.vec_blocks, kVecThreads, 0, op.stream>>>(op.g, ms.v.patch32, x, op.d_mask,
+    gather_kernel<float><<<op.vec_blocks, kVecThreads, 0, op.stream>>>(op.g, brick_tiles(op.g), ms.v.patch32, x, op.d_mask,
                                                                        op.mask_mode, op.extra32(), y, nullptr, nullptr);
     ICC_CUDA(cudaGetLastError(), "tc apply launch");
     return ICC_OK;
@@ -1574,7 +1574,7 @@ int mixed_profile_apply(Op &op, const float *x, float *y, int reps, double *cont
         ICC_CUDA(launch_apply_tc(op.stream, ms.d_inst, 1, op.g.nbricks, ms.d_desc, ms.d_bmat, ms.d_err, op.num_sms),
                  "tc apply launch");
         cudaEventRecord(ev[3 * r + 1], op.stream);
-        gather_kernel<float><<<op.vec_blocks, kVecThreads, 0, op.stream>>>(op.g, ms.v.patch32, x, op.d_mask,
+        gather_kernel<float><<<op.vec_blocks, kVecThreads, 0, op.stream>>>(op.g, brick_tiles(op.g), ms.v.patch32, x, op.d_mask,
                                                                            ICC_MASK_NONE, op.extra32(), y, nullptr,
                                                                            nullptr);
         cudaEventRecord(ev[3 * r + 2], op.stream);

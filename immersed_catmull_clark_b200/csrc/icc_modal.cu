@@ -1,0 +1,286 @@
+// Host side of the operator in Legendre modes (icc_modal.cuh): the test whether a handle's element
+// matrices have that form, the choice of the tile, and the launches.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "icc_device.cuh"
+#include "icc_vec.cuh"
+#include "icc_modal.cuh"
+
+namespace icc {
+
+// ---- set-up ---------------------------------------------------------------------------------------
+
+namespace {
+
+// M <- (Az (x) Ay (x) Ax per component) M for 3 x 3 matrices (row-major): rows of M (81 x 81) combined one
+// direction after the other
+void rows_by(const double *Ax, const double *Ay, const double *Az, double *M) {
+    const double *A[3] = {Ax, Ay, Az};
+    const int st[3] = {1, 3, 9};
+    for (int d = 0; d < 3; ++d)
+        for (int i = 0; i < 81; ++i) {
+            if ((i % 27) / st[d] % 3 != 0) continue;
+            double *r0 = M + i * 81, *r1 = r0 + st[d] * 81, *r2 = r1 + st[d] * 81;
+            const double *a = A[d];
+            for (int j = 0; j < 81; ++j) {
+                const double u = r0[j], v = r1[j], w = r2[j];
+                r0[j] = a[0] * u + a[1] * v + a[2] * w;
+                r1[j] = a[3] * u + a[4] * v + a[5] * w;
+                r2[j] = a[6] * u + a[7] * v + a[8] * w;
+            }
+        }
+}
+
+// out = L K L' with L = Az (x) Ay (x) Ax per component (81 x 81, row-major)
+void congruence(const double *Ax, const double *Ay, const double *Az, const double *K, double *out) {
+    double t[81 * 81];
+    std::memcpy(t, K, sizeof(t));
+    rows_by(Ax, Ay, Az, t);
+    for (int i = 0; i < 81; ++i)
+        for (int j = 0; j < 81; ++j) out[j * 81 + i] = t[i * 81 + j];
+    rows_by(Ax, Ay, Az, out);
+    for (int i = 0; i < 81; ++i)
+        for (int j = 0; j < i; ++j) std::swap(out[i * 81 + j], out[j * 81 + i]);
+}
+
+}  // namespace
+
+// The element's B-splines in terms of the translated ones, N = R B: R of an element whose end factors
+// are a (first control value) and b (last): N_0 = a B_0, N_2 = b B_2, N_1 = B_1 + (1 - a) B_0 + (1 - b) B_2.
+static void end_matrix(double a, double b, double r[9]) {
+    const double m[9] = {a, 0.0, 0.0, 1.0 - a, 1.0, 1.0 - b, 0.0, 0.0, b};
+    std::memcpy(r, m, sizeof(m));
+}
+
+bool modal_setup(const Op &op, ModalHost &m) {
+    m.ok = false;
+    const Geom &g = op.g;
+    const int n[3] = {g.nx, g.ny, g.nz};
+    if (op.ndof >= (1LL << 31) || op.nel >= (1LL << 31)) return false;   // 32-bit indices in the kernels
+    // end factors of every 1-D type, from its basis values at the three Gauss points
+    const double xg[3] = {-std::sqrt(0.6), 0.0, std::sqrt(0.6)};
+    double bu[9];
+    for (int q = 0; q < 3; ++q) {
+        const double t = 0.5 * (xg[q] + 1.0);
+        bu[q] = 0.5 * (1.0 - t) * (1.0 - t);
+        bu[3 + q] = 0.5 + t - t * t;
+        bu[6 + q] = 0.5 * t * t;
+    }
+    for (int d = 0; d < 3; ++d) {
+        if ((int)op.host_type1d[d].size() != n[d] || op.host_basis1d[d].empty()) return false;
+        m.a[d] = m.b[d] = 1.0;
+        for (int e = 0; e < n[d]; ++e) {
+            const auto &v = op.host_basis1d[d][(size_t)op.host_type1d[d][(size_t)e]];
+            const double a = std::round(v[1] / bu[1]), b = std::round(v[7] / bu[7]);
+            double r[9];
+            end_matrix(a, b, r);
+            for (int i = 0; i < 3; ++i)
+                for (int q = 0; q < 3; ++q) {
+                    const double w = r[3 * i] * bu[q] + r[3 * i + 1] * bu[3 + q] + r[3 * i + 2] * bu[6 + q];
+                    if (!(std::fabs(w - v[(size_t)(3 * i + q)]) <= 1e-12)) return false;
+                }
+            if ((a != 1.0 && e != 0) || (b != 1.0 && e != n[d] - 1)) return false;
+            if (e == 0) m.a[d] = a;
+            if (e == n[d] - 1) m.b[d] = b;
+        }
+    }
+    // the (element type, position class) pairs that occur; class 0 interior, 1 first, 2 last, 3 both
+    std::vector<uint8_t> seen((size_t)op.ntypes * 64, 0);
+    std::vector<long long> count((size_t)op.ntypes, 0);
+    auto cls = [&](int d, int e) { return (e == 0 ? 1 : 0) | (e == n[d] - 1 ? 2 : 0); };
+    for (int ez = 0, e = 0; ez < g.nz; ++ez)
+        for (int ey = 0; ey < g.ny; ++ey) {
+            const int cyz = 4 * cls(1, ey) + 16 * cls(2, ez);
+            for (int ex = 0; ex < g.nx; ++ex, ++e) {
+                const int t = op.host_type_id[(size_t)e];
+                seen[(size_t)t * 64 + cls(0, ex) + cyz] = 1;
+                count[(size_t)t]++;
+            }
+        }
+    auto matrix_of = [&](int c, double R[3][9], bool inverse) {
+        for (int d = 0; d < 3; ++d) {
+            const int k = c >> (2 * d) & 3;
+            const double a = k & 1 ? m.a[d] : 1.0, b = k & 2 ? m.b[d] : 1.0;
+            if (!inverse) {
+                end_matrix(a, b, R[d]);
+            } else {
+                const double w[9] = {1.0 / a, 0.0, 0.0, (a - 1.0) / a, 1.0, (b - 1.0) / b, 0.0, 0.0, 1.0 / b};
+                std::memcpy(R[d], w, sizeof(w));
+            }
+        }
+    };
+    // the uniform matrix from the most frequent type, then its modes
+    int mt = 0;
+    for (int t = 1; t < op.ntypes; ++t)
+        if (count[(size_t)t] > count[(size_t)mt]) mt = t;
+    int mc = 0;
+    while (!seen[(size_t)mt * 64 + mc]) ++mc;
+    std::vector<double> ku(81 * 81), kl(81 * 81), kp(81 * 81, 0.0), kt(81 * 81);
+    double R[3][9];
+    matrix_of(mc, R, true);
+    congruence(R[0], R[1], R[2], op.host_ktypes.data() + (size_t)mt * 81 * 81, ku.data());
+    // rows: control values (u0, u1, u2) of the modes mean, slope, curvature
+    const double sh[9] = {1.0, 1.0, 1.0, -0.5, 0.0, 0.5, 1.0 / 3.0, -1.0 / 6.0, 1.0 / 3.0};
+    const double shinv_t[9] = {1.0 / 6.0, -1.0, 1.0, 2.0 / 3.0, 0.0, -2.0, 1.0 / 6.0, 1.0, 1.0};   // T', modes = T u
+    congruence(sh, sh, sh, ku.data(), kl.data());
+    const int pw[3] = {1, 3, 9};
+    for (int c = 0; c < 3; ++c)
+        for (int i = 0; i < 27; ++i) {
+            const int r = c * 27 + i;
+            m.diag[c][i] = i ? kl[(size_t)r * 81 + r] : 0.0;
+            kp[(size_t)r * 81 + r] = m.diag[c][i];
+        }
+    std::memset(m.off, 0, sizeof(m.off));
+    for (int A = 0; A < 3; ++A)
+        for (int B = A + 1; B < 3; ++B)
+            for (int i = 0; i < 27; ++i) {
+                const int ia = i / pw[A] % 3, ib = i / pw[B] % 3, k = i / pw[3 - A - B] % 3, p = A + B - 1;
+                for (int q = 0; q < 2; ++q) {
+                    const bool on = q == 0 ? (ia >= 1 && ib <= 1) : (ia <= 1 && ib >= 1);
+                    if (!on) continue;
+                    const int r = A * 27 + i, s = B * 27 + (q == 0 ? i - pw[A] + pw[B] : i + pw[A] - pw[B]);
+                    const double v = 0.5 * (kl[(size_t)r * 81 + s] + kl[(size_t)s * 81 + r]);
+                    m.off[p][q][q == 0 ? 2 * (ia - 1) + ib : 2 * ia + ib - 1][k] = v;
+                    kp[(size_t)r * 81 + s] = kp[(size_t)s * 81 + r] = v;
+                }
+            }
+    // every matrix that occurs must be the one of these entries, seen through its element's basis.  The
+    // knots i/n round, so even exact integration leaves n eps of an element's size in its matrix.
+    congruence(shinv_t, shinv_t, shinv_t, kp.data(), ku.data());
+    double kmax = 0.0;
+    for (double v : ku) kmax = std::fmax(kmax, std::fabs(v));
+    const double tol = 4.0 * 2.220446049250313e-16 * (64.0 + std::max(n[0], std::max(n[1], n[2]))) * kmax;
+    for (int t = 0; t < op.ntypes; ++t)
+        for (int c = 0; c < 64; ++c) {
+            if (!seen[(size_t)t * 64 + c]) continue;
+            matrix_of(c, R, false);
+            congruence(R[0], R[1], R[2], ku.data(), kt.data());
+            const double *K = op.host_ktypes.data() + (size_t)t * 81 * 81;
+            double rmax = 1.0;   // N = R B stretches the matrix of an end element
+            for (int d = 0; d < 3; ++d) rmax *= std::fmax(R[d][0], R[d][8]) * std::fmax(R[d][0], R[d][8]);
+            for (int i = 0; i < 81 * 81; ++i)
+                if (!(std::fabs(kt[(size_t)i] - K[i]) <= tol * rmax)) return false;
+        }
+    m.kunif = ku;
+    m.ok = true;
+    return true;
+}
+
+// ---- the tile ------------------------------------------------------------------------------------
+
+// Columns of a tile (threads), its extent and length, by a model of the launch: clocks of a CTA's march
+// (per warp and step, for planes and for elements, measured with the kernel alone on the chip) times the
+// waves of CTAs.  Short marches of small tiles fill the chip on small grids, where latency counts;
+// 256 columns waste the least on the two extra planes of a tile and on its overlap.
+template <class T>
+ModalTile modal_tile(const Geom &g, int num_sms) {
+    const bool f64 = sizeof(T) == 8;
+    const double c_el = f64 ? 1500.0 : 700.0, c_pl = f64 ? 700.0 : 400.0, c_step = 500.0, c_start = 2500.0;
+    ModalTile best;
+    double cost = INFINITY;
+    struct Shape { int nt, ltx, per_sm; };
+    // FP64: 256 columns' state fills tensor memory; FP32: 512
+    const Shape f64_shapes[] = {{256, 5, 1}, {256, 4, 1}, {64, 4, 2}, {64, 3, 2}};
+    const Shape f32_shapes[] = {{512, 5, 1}, {512, 4, 1}, {64, 4, 4}, {64, 3, 4}};
+    const Shape (&shapes)[4] = f64 ? f64_shapes : f32_shapes;
+    for (const Shape &s : shapes) {
+        const int tx = 1 << s.ltx, rows = s.nt >> s.ltx;
+        if (tx > 8 && tx >= 2 * g.nx) continue;
+        for (int nty = (g.ny + rows - 1) / rows, k = 0; k < 3; ++k, ++nty) {
+            const int ty = (g.ny + nty - 1) / nty;
+            if (ty < 2 && g.ny > 1) break;
+            for (int ntz = 1; ntz <= g.nz; ++ntz) {
+                const int tz = (g.nz + ntz - 1) / ntz;
+                if (tz < 2 && g.nz > 1) break;
+                const long long n = (long long)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty) * ((g.nz + tz - 1) / tz);
+                const long long slots = (long long)num_sms * s.per_sm, waves = (n + slots - 1) / slots;
+                const long long on_sm = std::min<long long>(s.per_sm, (n + num_sms - 1) / num_sms);
+                const double warps = std::max(1.0, (double)on_sm * s.nt / 128.0);   // per scheduler
+                const double march = warps * (tz * c_el + (tz + 2) * c_pl) + (tz + 5) * c_step;
+                const double c = waves * march + c_start;
+                if (c < cost) {
+                    cost = c;
+                    best.nt = s.nt;
+                    best.t = make_tiles(g.nx, g.ny, g.nz, tx, ty, tz);
+                }
+            }
+        }
+    }
+    return best;
+}
+template ModalTile modal_tile<double>(const Geom &g, int num_sms);
+template ModalTile modal_tile<float>(const Geom &g, int num_sms);
+
+// ---- launches -------------------------------------------------------------------------------------
+
+template <class T>
+ModalK<T> modal_entries(const ModalHost &m) {
+    ModalK<T> k;
+    for (int c = 0; c < 3; ++c)
+        for (int i = 0; i < 27; ++i) k.diag[c][i] = T(m.diag[c][i]);
+    for (int p = 0; p < 3; ++p)
+        for (int q = 0; q < 2; ++q)
+            for (int n = 0; n < 4; ++n)
+                for (int l = 0; l < 3; ++l) k.off[p][q][n][l] = T(m.off[p][q][n][l]);
+    return k;
+}
+template ModalK<double> modal_entries<double>(const ModalHost &m);
+template ModalK<float> modal_entries<float>(const ModalHost &m);
+
+template <class T, int NT, bool PCG, bool MANY>
+static cudaError_t launch_one(cudaStream_t s, const ModalK<T> &K, const ModalSys<T> &one, const ModalSys<T> *many,
+                              const int2 *list, int ntiles, int ltx) {
+    const size_t smem = modal_smem<T>(NT, ltx, ModalCfg<T, NT>::slots, PCG);
+    const cudaError_t e = cudaFuncSetAttribute(modal_apply_kernel<T, NT, PCG, MANY>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+    if (e != cudaSuccess) return e;
+    modal_apply_kernel<T, NT, PCG, MANY><<<ntiles, NT, smem, s>>>(K, one, many, list);
+    return cudaGetLastError();
+}
+
+template <class T>
+cudaError_t launch_modal_apply(cudaStream_t s, const ModalK<T> &K, const ModalSys<T> &one, const ModalSys<T> *many,
+                               const int2 *list, int ntiles, int nt, int ltx, bool pcg) {
+    constexpr int kWide = sizeof(T) == 8 ? 256 : 512;
+    if (nt == kWide) {
+        if (many) return launch_one<T, kWide, true, true>(s, K, one, many, list, ntiles, ltx);
+        return pcg ? launch_one<T, kWide, true, false>(s, K, one, many, list, ntiles, ltx)
+                   : launch_one<T, kWide, false, false>(s, K, one, many, list, ntiles, ltx);
+    }
+    if (many) return launch_one<T, 64, true, true>(s, K, one, many, list, ntiles, ltx);
+    return pcg ? launch_one<T, 64, true, false>(s, K, one, many, list, ntiles, ltx)
+               : launch_one<T, 64, false, false>(s, K, one, many, list, ntiles, ltx);
+}
+template cudaError_t launch_modal_apply<double>(cudaStream_t, const ModalK<double> &, const ModalSys<double> &,
+                                                const ModalSys<double> *, const int2 *, int, int, int, bool);
+template cudaError_t launch_modal_apply<float>(cudaStream_t, const ModalK<float> &, const ModalSys<float> &,
+                                               const ModalSys<float> *, const int2 *, int, int, int, bool);
+
+// The grid part of a system's entry.
+template <class T>
+ModalSys<T> modal_sys(const Op &op, const ModalTile &t) {
+    ModalSys<T> S;
+    std::memset((void *)&S, 0, sizeof(S));
+    const Geom &g = op.g;
+    S.nx = g.nx; S.ny = g.ny; S.nz = g.nz;
+    S.cx = g.cx; S.cy = g.cy; S.cz = g.cz;
+    S.nsc = (int)g.nsc;
+    S.t = t.t;
+    for (int d = 0; d < 3; ++d) {
+        S.a[d] = T(op.modal.a[d]);
+        S.b[d] = T(op.modal.b[d]);
+    }
+    S.kfac = T(1);
+    S.mask = op.d_mask;
+    S.mask_mode = op.mask_mode;
+    return S;
+}
+template ModalSys<double> modal_sys<double>(const Op &op, const ModalTile &t);
+template ModalSys<float> modal_sys<float>(const Op &op, const ModalTile &t);
+
+}  // namespace icc

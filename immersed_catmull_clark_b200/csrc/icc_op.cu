@@ -30,6 +30,7 @@
 #include "icc_internal.h"
 #include "icc_device.cuh"
 #include "icc_vec.cuh"
+#include "icc_modal.cuh"
 
 namespace icc {
 
@@ -278,9 +279,57 @@ int Op::init(const Space &s, const double *ke_types, int nt, const int32_t *type
     ICC_CUDA(cudaEventCreate(&ev0), "cudaEventCreate");
     ICC_CUDA(cudaEventCreate(&ev1), "cudaEventCreate");
 
+    std::vector<double> kd((size_t)nt * 81);
+    for (int t = 0; t < nt; ++t)
+        for (int a = 0; a < 81; ++a) kd[(size_t)t * 81 + a] = ke_types[((size_t)t * 81 + a) * 81 + a];
+    host_ktypes.assign(ke_types, ke_types + (size_t)nt * 81 * 81);
+    int rc;
+    if ((rc = dev_alloc(&d_kdiag, kd.size(), "alloc kdiag"))) return rc;
+    ICC_CUDA(cudaMemcpyAsync(d_kdiag, kd.data(), kd.size() * 8, cudaMemcpyHostToDevice, stream), "copy kdiag");
+    if ((rc = dev_alloc(&d_type_id, (size_t)nel, "alloc type_id"))) return rc;
+    ICC_CUDA(cudaMemcpyAsync(d_type_id, type_id, (size_t)nel * 4, cudaMemcpyHostToDevice, stream), "copy type_id");
+    host_type_id.assign(type_id, type_id + nel);
+    for (int d = 0; d < 3; ++d) {
+        host_type1d[d] = s.type1d[d];
+        host_basis1d[d] = s.basis1d[d];
+    }
+    // every set-up copy is ordered on the handle's stream (a non-blocking stream is not ordered
+    // after copies on the legacy default stream); the host arrays must outlive them
+    ICC_CUDA(cudaStreamSynchronize(stream), "set-up copies");
+    if (modal_setup(*this, modal)) {
+        mtile = modal_tile<double>(g, num_sms);
+        tiles = mtile.t;
+    } else {
+        tiles = brick_tiles(g);
+        if ((rc = init_dense())) return rc;
+    }
+
+    if ((rc = dev_alloc(&d_scale, (size_t)nel, "alloc scale"))) return rc;
+    if ((rc = dev_alloc(&d_mask, (size_t)ndof, "alloc mask"))) return rc;
+    if ((rc = dev_alloc(&d_patch, (size_t)tiles.n * tiles.vol, "alloc patch scratch"))) return rc;
+    if ((rc = dev_alloc(&d_x_in, (size_t)ndof, "alloc io"))) return rc;
+    if ((rc = dev_alloc(&d_y_out, (size_t)ndof, "alloc io"))) return rc;
+    vec_blocks = num_sms * 4;
+    if ((rc = dev_alloc(&d_partials, (size_t)vec_blocks * 2, "alloc partials"))) return rc;
+    if ((rc = dev_alloc(&d_state, 1, "alloc state"))) return rc;
+    if ((rc = dev_alloc(&d_counter, 1, "alloc counter"))) return rc;
+    ICC_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned), stream), "clear counter");
+    ICC_CUDA(cudaStreamSynchronize(stream), "clear counter");
+    ICC_CUDA(cudaMallocHost((void **)&h_state, sizeof(PcgState)), "alloc pinned state");
+    if ((rc = set_scale(scale))) return rc;
+    if ((rc = set_mask(free_mask, mode))) return rc;
+    return ICC_OK;
+}
+
+// Data of the dense FP64 contraction: the element matrices as DMMA fragments and the tile plan.
+int Op::init_dense() {
+    const double *ke_types = host_ktypes.data();
+    const int nt = ntypes;
+    const int32_t *type_id = host_type_id.data();
+    int rc;
     // element matrices in DMMA B-fragment order: kfrag[t][ks][nt][lane] = K[n][k] with
     // k = 4 ks + lane % 4 (trial), n = 8 nt + lane / 4 (test); zero outside 81 x 81.
-    std::vector<double> kf((size_t)nt * kFragPerType, 0.0), kd((size_t)nt * 81);
+    std::vector<double> kf((size_t)nt * kFragPerType, 0.0);
     for (int t = 0; t < nt; ++t) {
         const double *K = ke_types + (size_t)t * 81 * 81;
         for (int ks = 0; ks < kKSteps; ++ks)
@@ -290,22 +339,9 @@ int Op::init(const Space &s, const double *ke_types, int nt, const int32_t *type
                     kf[(size_t)t * kFragPerType + (ks * kNTiles + ntile) * 32 + lane] =
                         (k < 81 && n < 81) ? K[n * 81 + k] : 0.0;
                 }
-        for (int a = 0; a < 81; ++a) kd[(size_t)t * 81 + a] = K[a * 81 + a];
     }
-    host_ktypes.assign(ke_types, ke_types + (size_t)nt * 81 * 81);
-    int rc;
     if ((rc = dev_alloc(&d_kfrag, kf.size(), "alloc kfrag"))) return rc;
-    if ((rc = dev_alloc(&d_kdiag, kd.size(), "alloc kdiag"))) return rc;
     ICC_CUDA(cudaMemcpyAsync(d_kfrag, kf.data(), kf.size() * 8, cudaMemcpyHostToDevice, stream), "copy kfrag");
-    ICC_CUDA(cudaMemcpyAsync(d_kdiag, kd.data(), kd.size() * 8, cudaMemcpyHostToDevice, stream), "copy kdiag");
-    if ((rc = dev_alloc(&d_type_id, (size_t)nel, "alloc type_id"))) return rc;
-    ICC_CUDA(cudaMemcpyAsync(d_type_id, type_id, (size_t)nel * 4, cudaMemcpyHostToDevice, stream), "copy type_id");
-    host_type_id.assign(type_id, type_id + nel);
-    for (int d = 0; d < 3; ++d) {
-        host_type1d[d] = s.type1d[d];
-        host_basis1d[d] = s.basis1d[d];
-    }
-
     // brick tile plan: per brick, its elements grouped by type (first-appearance order) and cut
     // into warp tiles of 16 (255 marks an empty row)
     std::vector<int> tstart(1, 0), ttype;
@@ -343,26 +379,9 @@ int Op::init(const Space &s, const double *ke_types, int nt, const int32_t *type
     ICC_CUDA(cudaMemcpyAsync(d_tile_start, tstart.data(), tstart.size() * 4, cudaMemcpyHostToDevice, stream), "copy tiles");
     ICC_CUDA(cudaMemcpyAsync(d_tile_type, ttype.data(), ttype.size() * 4, cudaMemcpyHostToDevice, stream), "copy tiles");
     ICC_CUDA(cudaMemcpyAsync(d_tile_elem, telem.data(), telem.size(), cudaMemcpyHostToDevice, stream), "copy tiles");
-    // every set-up copy is ordered on the handle's stream (a non-blocking stream is not ordered
-    // after copies on the legacy default stream); the host arrays must outlive them
     ICC_CUDA(cudaStreamSynchronize(stream), "set-up copies");
-
-    if ((rc = dev_alloc(&d_scale, (size_t)nel, "alloc scale"))) return rc;
-    if ((rc = dev_alloc(&d_mask, (size_t)ndof, "alloc mask"))) return rc;
-    if ((rc = dev_alloc(&d_patch, (size_t)g.nbricks * 3 * kPVol, "alloc patch scratch"))) return rc;
-    if ((rc = dev_alloc(&d_x_in, (size_t)ndof, "alloc io"))) return rc;
-    if ((rc = dev_alloc(&d_y_out, (size_t)ndof, "alloc io"))) return rc;
-    vec_blocks = num_sms * 4;
-    if ((rc = dev_alloc(&d_partials, (size_t)vec_blocks * 2, "alloc partials"))) return rc;
-    if ((rc = dev_alloc(&d_state, 1, "alloc state"))) return rc;
-    if ((rc = dev_alloc(&d_counter, 1, "alloc counter"))) return rc;
-    ICC_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned), stream), "clear counter");
-    ICC_CUDA(cudaStreamSynchronize(stream), "clear counter");
-    ICC_CUDA(cudaMallocHost((void **)&h_state, sizeof(PcgState)), "alloc pinned state");
     ICC_CUDA(cudaFuncSetAttribute(apply_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kApplySmem),
              "cudaFuncSetAttribute");
-    if ((rc = set_scale(scale))) return rc;
-    if ((rc = set_mask(free_mask, mode))) return rc;
     return ICC_OK;
 }
 
@@ -475,20 +494,33 @@ int Op::set_extra(int64_t count, const int64_t *rows, const int64_t *cols, const
     return ICC_OK;
 }
 
+// The FP64 contraction of x into the tile partial sums.
+cudaError_t Op::enqueue_contract(cudaStream_t s, const double *x, const PcgState *st) {
+    if (modal.ok) {
+        ModalSys<double> S = modal_sys<double>(*this, mtile);
+        S.scale = d_scale;
+        S.x = x;
+        S.patch = d_patch;
+        S.st = const_cast<PcgState *>(st);
+        return launch_modal_apply<double>(s, modal_entries<double>(modal), S, nullptr, nullptr, tiles.n, mtile.nt,
+                                          tiles.ltx, false);
+    }
+    apply_f64_kernel<<<g.nbricks, kApplyThreads, kApplySmem, s>>>(g, x, d_mask, mask_mode != ICC_MASK_NONE, d_scale,
+                                                                   d_kfrag, d_tile_start, d_tile_type, d_tile_elem,
+                                                                   d_patch, st);
+    return cudaGetLastError();
+}
+
 // Enqueue y = A x on the op's stream (FP64).  partials != null also forms p'y per CTA.
 void Op::enqueue_apply(const double *x, double *y, double *partials, const PcgState *st) {
-    apply_f64_kernel<<<g.nbricks, kApplyThreads, kApplySmem, stream>>>(
-        g, x, d_mask, mask_mode != ICC_MASK_NONE, d_scale, d_kfrag, d_tile_start, d_tile_type, d_tile_elem, d_patch,
-        st);
-    gather_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(g, d_patch, x, d_mask, mask_mode, extra64(), y,
+    enqueue_contract(stream, x, st);
+    gather_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(g, tiles, d_patch, x, d_mask, mask_mode, extra64(), y,
                                                                   partials, st);
 }
 
 void Op::enqueue_apply_on(cudaStream_t s, const double *x, double *y) {
-    apply_f64_kernel<<<g.nbricks, kApplyThreads, kApplySmem, s>>>(
-        g, x, d_mask, mask_mode != ICC_MASK_NONE, d_scale, d_kfrag, d_tile_start, d_tile_type, d_tile_elem, d_patch,
-        nullptr);
-    gather_kernel<double><<<vec_blocks, kVecThreads, 0, s>>>(g, d_patch, x, d_mask, mask_mode, extra64(), y,
+    enqueue_contract(s, x, nullptr);
+    gather_kernel<double><<<vec_blocks, kVecThreads, 0, s>>>(g, tiles, d_patch, x, d_mask, mask_mode, extra64(), y,
                                                              nullptr, nullptr);
 }
 
@@ -528,10 +560,8 @@ int Op::ensure_pcg_buffers() {
 // harmlessly.
 void Op::enqueue_pcg_iteration() {
     pcg_p_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(ndof, d_r, d_inv, d_p, d_state);
-    apply_f64_kernel<<<g.nbricks, kApplyThreads, kApplySmem, stream>>>(
-        g, d_p, d_mask, mask_mode != ICC_MASK_NONE, d_scale, d_kfrag, d_tile_start, d_tile_type, d_tile_elem, d_patch,
-        d_state);
-    gather_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(g, d_patch, d_p, d_mask, mask_mode, extra64(), d_ap,
+    enqueue_contract(stream, d_p, d_state);
+    gather_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(g, tiles, d_patch, d_p, d_mask, mask_mode, extra64(), d_ap,
                                                                   d_partials,
                                                                   d_state, d_state, d_counter);
     pcg_update_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(ndof, d_p, d_ap, d_inv, d_x, d_r, d_partials,
@@ -861,12 +891,10 @@ int icc_op_profile_apply(icc_op *op, const double *x_dev, double *y_dev, int32_t
     for (auto &e : ev) ICC_CUDA(cudaEventCreate(&e), "event create");
     for (int r = 0; r < reps; ++r) {
         cudaEventRecord(ev[3 * r], o.stream);
-        icc::apply_f64_kernel<<<o.g.nbricks, icc::kApplyThreads, icc::kApplySmem, o.stream>>>(
-            o.g, x_dev, o.d_mask, o.mask_mode != ICC_MASK_NONE, o.d_scale, o.d_kfrag, o.d_tile_start, o.d_tile_type,
-            o.d_tile_elem, o.d_patch, nullptr);
+        ICC_CUDA(o.enqueue_contract(o.stream, x_dev, nullptr), "apply launch");
         cudaEventRecord(ev[3 * r + 1], o.stream);
         icc::gather_kernel<double><<<o.vec_blocks, icc::kVecThreads, 0, o.stream>>>(
-            o.g, o.d_patch, x_dev, o.d_mask, o.mask_mode, o.extra64(), y_dev, nullptr, nullptr);
+            o.g, o.tiles, o.d_patch, x_dev, o.d_mask, o.mask_mode, o.extra64(), y_dev, nullptr, nullptr);
         cudaEventRecord(ev[3 * r + 2], o.stream);
     }
     cudaError_t e = cudaEventSynchronize(ev.back());

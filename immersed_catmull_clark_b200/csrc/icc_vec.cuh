@@ -25,6 +25,44 @@ __device__ __forceinline__ int node_bricks(int j, int B, int nb, int *bi, int *l
     return 1;
 }
 
+// The same for a tile cut: the last tile (b) that holds control point j along a direction, its index
+// there (l), and whether the tile before holds it too (at index l + B).
+struct TileAt {
+    int b, l;
+    bool two;
+};
+__device__ __forceinline__ TileAt tile_at(int j, const FastDiv &d, int B, int nb) {
+    TileAt t;
+    t.b = min(j / d, nb - 1);
+    t.l = j - t.b * B;
+    t.two = t.l <= 1 && t.b >= 1;
+    return t;
+}
+
+// The <= 8 tile partials of control point (ix; ty, tz along y and z) summed in a fixed order: lower
+// tiles first along z, then y, then x.
+template <class T>
+__device__ __forceinline__ void tile_sum(const Tiles &t, const T *__restrict__ patch, int ix, const TileAt &ty,
+                                         const TileAt &tz, T (&sv)[3]) {
+    const TileAt tx = tile_at(ix, t.dx, t.tx, t.ntx);
+    const int row = t.tx + 2, plane = row * (t.ty + 2), comp = plane * (t.tz + 2);
+    sv[0] = sv[1] = sv[2] = T(0);
+    for (int a = tz.two ? 0 : 1; a < 2; ++a)
+        for (int q = ty.two ? 0 : 1; q < 2; ++q) {
+            const size_t tile = (size_t)tx.b + (size_t)t.ntx * ((ty.b - 1 + q) + (size_t)t.nty * (tz.b - 1 + a));
+            const T *pb = patch + tile * (size_t)t.vol + (a ? tz.l : tz.l + t.tz) * plane + (q ? ty.l : ty.l + t.ty) * row + tx.l;
+            if (tx.two) {
+                const T *pl = pb - t.vol + t.tx;
+                sv[0] += pl[0];
+                sv[1] += pl[comp];
+                sv[2] += pl[2 * comp];
+            }
+            sv[0] += pb[0];
+            sv[1] += pb[comp];
+            sv[2] += pb[2 * comp];
+        }
+}
+
 // ---- PCG scalar steps (rust/src/solver.rs:41-71), run by one thread ---------------------------
 
 // p'Ap -> alpha, or breakdown (rust/src/solver.rs:41-51)
@@ -48,44 +86,26 @@ __device__ __forceinline__ void pcg_beta_step(PcgState *st, double rr, double rz
         st->beta = rz / st->rz_old;
         st->rz_old = rz;
         if (st->iter >= st->max_iter) st->status = kStatMaxIter;
+        else if (st->repl_delta > 0.0 && st->iter % st->repl_every == 0 &&
+                 (res < st->repl_delta * st->repl_res || st->iter - st->repl_iter >= st->repl_seg))
+            st->status = kStatReplace;
     }
 }
 
 // True in exactly one CTA: the last to finish.  Every CTA has stored its partial before calling;
 // the last one then reads all partials (in fixed order, so the result does not depend on which
 // CTA is last) and resets the counter for the next use.
-__device__ __forceinline__ bool last_block(unsigned *counter) {
+__device__ __forceinline__ bool last_block(unsigned *counter, unsigned total) {
     __shared__ bool is_last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) is_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) is_last = atomicAdd(counter, 1u) == total - 1u;
     __syncthreads();
     if (is_last) {
         __threadfence();
         if (threadIdx.x == 0) *counter = 0u;
     }
     return is_last;
-}
-
-// The <= 8 brick partials of control point (ix, iy, iz) summed in a fixed order (lower bricks
-// first along z, then y, then x).
-template <class T>
-__device__ __forceinline__ void node_partials(const Geom &g, const T *__restrict__ patch, int ix, int iy, int iz, T &s0,
-                                              T &s1, T &s2) {
-    int bx[2], lx[2], by[2], ly[2], bz[2], lz[2];
-    const int nbx = node_bricks(ix, kBX, g.nbx, bx, lx);
-    const int nby = node_bricks(iy, kBY, g.nby, by, ly);
-    const int nbz = node_bricks(iz, kBZ, g.nbz, bz, lz);
-    s0 = s1 = s2 = T(0);
-    for (int a = 0; a < nbz; ++a)
-        for (int q = 0; q < nby; ++q)
-            for (int w = 0; w < nbx; ++w) {
-                const size_t brick = (size_t)bx[w] + (size_t)g.nbx * (by[q] + (size_t)g.nby * bz[a]);
-                const T *pb = patch + brick * 3 * kPVol + (lz[a] * kPY + ly[q]) * kPX + lx[w];
-                s0 += pb[0];
-                s1 += pb[kPVol];
-                s2 += pb[2 * kPVol];
-            }
 }
 
 // Row idx of the sparse term applied to the masked input: sum_k S[idx][k] (m .* p)[k].
@@ -102,12 +122,12 @@ __device__ __forceinline__ T sparse_row(const Sparse<T> &sp, long long idx, cons
     return acc;
 }
 
-// y = sum of the brick partials of each node (fixed order) plus the sparse term, output mask
+// y = sum of the tile partials of each node (fixed order) plus the sparse term, output mask
 // applied; optionally the CTA partial of p'y (in double), and with `fuse` the alpha step in the
 // last CTA.
 template <class T>
 __global__ void __launch_bounds__(kVecThreads)
-gather_kernel(Geom g, const T *__restrict__ patch, const T *__restrict__ p, const uint8_t *__restrict__ mask,
+gather_kernel(Geom g, Tiles t, const T *__restrict__ patch, const T *__restrict__ p, const uint8_t *__restrict__ mask,
               int mask_mode, Sparse<T> sp, T *__restrict__ y, double *__restrict__ partials, const PcgState *st,
               PcgState *fuse = nullptr, unsigned *counter = nullptr) {
     if (st && st->status != 0) return;
@@ -119,24 +139,11 @@ gather_kernel(Geom g, const T *__restrict__ patch, const T *__restrict__ p, cons
     const int wstride = (gridDim.x * blockDim.x) >> 5;
     for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += wstride) {
         const int iy = row % g.cy, iz = row / g.cy;
-        int by[2], ly[2], bz[2], lz[2];
-        const int nby = node_bricks(iy, kBY, g.nby, by, ly);
-        const int nbz = node_bricks(iz, kBZ, g.nbz, bz, lz);
+        const TileAt ty = tile_at(iy, t.dy, t.ty, t.nty), tz = tile_at(iz, t.dz, t.tz, t.ntz);
         for (int ix = lane; ix < g.cx; ix += 32) {
             const long long n = (long long)row * g.cx + ix;
-            int bx[2], lx[2];
-            const int nbx = node_bricks(ix, kBX, g.nbx, bx, lx);
-            T s0 = T(0), s1 = T(0), s2 = T(0);
-            for (int a = 0; a < nbz; ++a)
-                for (int q = 0; q < nby; ++q)
-                    for (int w = 0; w < nbx; ++w) {
-                        size_t brick = (size_t)bx[w] + (size_t)g.nbx * (by[q] + (size_t)g.nby * bz[a]);
-                        const T *pb = patch + brick * 3 * kPVol + (lz[a] * kPY + ly[q]) * kPX + lx[w];
-                        s0 += pb[0];
-                        s1 += pb[kPVol];
-                        s2 += pb[2 * kPVol];
-                    }
-            T sv[3] = {s0, s1, s2};
+            T sv[3];
+            tile_sum(t, patch, ix, ty, tz, sv);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 long long idx = (long long)c * g.nsc + n;
@@ -152,7 +159,7 @@ gather_kernel(Geom g, const T *__restrict__ patch, const T *__restrict__ p, cons
     if (partials) {
         dot = block_sum(dot);
         if (threadIdx.x == 0) partials[blockIdx.x] = dot;
-        if (fuse && last_block(counter)) {
+        if (fuse && last_block(counter, gridDim.x)) {
             double s2 = 0.0;
             for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x) s2 += __ldcg(partials + i);
             s2 = block_sum(s2);
@@ -224,7 +231,7 @@ pcg_update_kernel(long long n, const T *__restrict__ p, const T *__restrict__ ap
         partials[2 * blockIdx.x] = rr;
         partials[2 * blockIdx.x + 1] = rz;
     }
-    if (fuse && last_block(counter)) {
+    if (fuse && last_block(counter, gridDim.x)) {
         double a = 0.0, c = 0.0;
         for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
             a += __ldcg(partials + 2 * i);

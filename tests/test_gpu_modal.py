@@ -1,0 +1,67 @@
+"""The operator in Legendre modes and the rule that chooses it.
+
+Isotropic element matrices take the sparse product in the element's Legendre modes, others the dense
+contraction.  Both are compared with the oracle's element loop at sizes around the tiles of either
+path (one element, tiles not filled, one more element than a tile, several tiles per direction)."""
+import numpy as np
+import pytest
+
+import immersed_catmull_clark_b200 as icc
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+APPLY_TOL = 1e-12       # FP64 parity bar of the repository
+APPLY_TOL_F32 = 5e-6    # FP32 parity bar of the repository
+
+SIZES = [(1, 1, 1), (2, 1, 3), (8, 8, 2), (9, 9, 3), (16, 16, 17), (17, 5, 33), (33, 16, 18), (31, 17, 9), (65, 33, 4),
+         (3, 40, 21), (40, 3, 2), (5, 2, 70)]
+
+
+def rel(a, b):
+    return np.linalg.norm(np.asarray(a) - np.asarray(b)) / max(np.linalg.norm(b), 1e-300)
+
+
+def oracle_apply(osp, types, tid, s, x, fm, mode):
+    fm = np.ones(len(x), dtype=np.uint8) if fm is None else fm
+    y = O.mf_apply(osp, types, tid.astype(np.int64), s, fm * x if mode != icc.MASK_NONE else x,
+                   np.ones(len(x), dtype=np.uint8), icc.MASK_NONE)
+    if mode == icc.MASK_ZERO:
+        return fm * y
+    return np.where(fm > 0, y, x) if mode == icc.MASK_IDENTITY else y
+
+
+@pytest.mark.parametrize("mode", [icc.MASK_NONE, icc.MASK_ZERO, icc.MASK_IDENTITY])
+@pytest.mark.parametrize("nel", SIZES)
+def test_modal_apply_matches_oracle(nel, mode):
+    bounds = ((-0.5, 2.0), (0.0, 0.7), (1.0, 2.3))   # elements of unequal sides
+    sp, osp = icc.SpaceBox(bounds, nel, 2), O.Space(bounds, nel, 2)
+    em = icc.elasticity_element_matrices(sp, *icc.lame(2.0, 0.25))
+    rng = np.random.default_rng(sum(nel) + mode)
+    s = rng.uniform(0.01, 1.0, sp.nel) ** 3
+    fm = None if mode == icc.MASK_NONE else (rng.uniform(size=sp.ndof) > 0.2).astype(np.uint8)
+    op = icc.MatrixFreeOperator(sp, em, s, fm, mode)
+    x = rng.standard_normal(sp.ndof)
+    y = op.matvec(x)
+    assert rel(y, oracle_apply(osp, em.types, em.type_id, s, x, fm, mode)) < APPLY_TOL
+    assert np.array_equal(y, op.matvec(x))           # bitwise reproducible
+    x32 = x.astype(np.float32)
+    ref = oracle_apply(osp, em.types, em.type_id, s, x32.astype(np.float64), fm, mode)
+    assert rel(op.matvec_f32(x32), ref) < APPLY_TOL_F32
+
+
+@pytest.mark.parametrize("nel", [(1, 1, 1), (9, 5, 6), (17, 9, 10)])
+def test_other_matrices_take_the_dense_path(nel):
+    """A perturbation of one part in 1e6 (symmetric or not) must show in the result: matrices that are
+    not exactly of the modal form are applied as they are given."""
+    bounds = ((0.0, 2.0), (0.0, 1.0), (0.0, 1.0))
+    sp, osp = icc.SpaceBox(bounds, nel, 2), O.Space(bounds, nel, 2)
+    em = icc.elasticity_element_matrices(sp, *icc.lame(1.0, 0.3))
+    rng = np.random.default_rng(7)
+    s = rng.uniform(0.1, 1.0, sp.nel)
+    x = rng.standard_normal(sp.ndof)
+    for sym in (True, False):
+        d = rng.standard_normal(em.types.shape) * 1e-6 * np.abs(em.types).max()
+        types = em.types + (0.5 * (d + d.transpose(0, 2, 1)) if sym else d)
+        op = icc.MatrixFreeOperator(sp, icc.ElementMatrices(types, em.type_id), s)
+        assert rel(op.matvec(x), oracle_apply(osp, types, em.type_id, s, x, None, icc.MASK_NONE)) < APPLY_TOL
