@@ -65,6 +65,7 @@ struct Tiles {
     int vol;                    // partial sums of a tile, three components
     FastDiv dx, dy, dz;         // division by tx, ty, tz
     FastDiv dcx, dcy;           // division by the control points of a row and of a column
+    FastDiv dntx, dnty;         // division by the tiles of a row and of a column
 };
 
 inline Tiles make_tiles(int nx, int ny, int nz, int tx, int ty, int tz) {
@@ -77,6 +78,7 @@ inline Tiles make_tiles(int nx, int ny, int nz, int tx, int ty, int tz) {
     t.vol = 3 * (tx + 2) * (ty + 2) * (tz + 2);
     t.dx = fast_div((unsigned)tx); t.dy = fast_div((unsigned)ty); t.dz = fast_div((unsigned)tz);
     t.dcx = fast_div((unsigned)nx + 2u); t.dcy = fast_div((unsigned)ny + 2u);
+    t.dntx = fast_div((unsigned)t.ntx); t.dnty = fast_div((unsigned)t.nty);
     return t;
 }
 
@@ -95,6 +97,7 @@ struct PcgState {
     double repl_res, repl_delta;
     long long repl_iter, repl_seg, repl_every;   // tested only when iter is a multiple of repl_every
     double rr_old;         // mixed form: r'r of the current residual
+    long long bars;        // modal form: barriers passed since the host cleared their counter
 };
 
 // A sparse term S added to the operator: CSR with 32-bit row pointers and columns over the
@@ -132,7 +135,7 @@ struct ModalHost {
     std::vector<double> kunif;
 };
 struct ModalTile {
-    int nt = 0;   // columns (threads) of a tile
+    int nt = 0;   // columns of a march; 0: cubes of 4 x 4 x 4 elements
     Tiles t{};
 };
 
@@ -175,6 +178,10 @@ struct Op {
     // PCG
     double *d_x = nullptr, *d_r = nullptr, *d_p = nullptr, *d_ap = nullptr, *d_inv = nullptr, *d_b = nullptr,
            *d_diag = nullptr, *d_partials = nullptr;
+    // modal form of the solve: its tile, the other direction, partial p'Ap, barrier counter, error flag
+    double *d_p2 = nullptr, *d_z = nullptr, *d_part_a = nullptr;
+    unsigned long long *d_bar = nullptr;
+    int *d_err = nullptr, *h_err = nullptr;
     PcgState *d_state = nullptr, *h_state = nullptr;
     unsigned *d_counter = nullptr;          // last-CTA counter of the fused reductions
     cudaGraphExec_t graph_exec = nullptr;
@@ -204,6 +211,7 @@ struct Op {
     int diagonal_dev(double *d);
     int ensure_pcg_buffers();
     void enqueue_pcg_iteration();
+    cudaError_t enqueue_pcg_modal(int iters);
     int pcg_fp64(const double *b, const double *diag, double tol, int64_t max_iter, int check_every, double *x,
                  int64_t *iters, double *rel_res);
 };
@@ -214,6 +222,8 @@ int cuda_fail(cudaError_t e, const char *where);
 bool modal_setup(const Op &op, ModalHost &m);
 template <class T>
 ModalTile modal_tile(const Geom &g, int num_sms);
+int modal_ctas(const Geom &g, const ModalTile &t, int num_sms);
+constexpr long long kGridWaitLimit = 1LL << 22;   // default polls of a grid barrier before it gives up
 
 // tensor-core mixed-precision path (icc_mixed.cu)
 void mixed_release(Op &op);

@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "icc_device.cuh"
+#include "icc_modal.cuh"
 #include "icc_tc.cuh"
 #include "icc_vec.cuh"
 
@@ -52,7 +53,6 @@ constexpr int kBFl = kTcN * kTcK;      // floats per B term
 constexpr uint32_t kBLbo = (kTcN / 8) * 128;  // bytes between K-adjacent core matrices of B
 constexpr uint32_t kSbo = 128;                // bytes between 8-row groups
 constexpr long long kWaitLimit = 1LL << 22;
-constexpr long long kGridWaitLimit = 1LL << 22;   // default polls of a grid barrier before it gives up
 
 // offset (floats) of element (row, k) in the canonical K-major no-swizzle layout with `rows` rows
 __host__ __device__ __forceinline__ int canon(int row, int k, int rows) {
@@ -105,10 +105,15 @@ struct VecSet {
     double *x64 = nullptr, *r64 = nullptr, *y64 = nullptr;
     double *part = nullptr;  // [9][tail CTAs]
     int part_cap = 0;
+    // modal form: the other direction, z = D^-1 r and the tile partial sums
+    float *p32b = nullptr, *z32 = nullptr, *mpatch = nullptr;
+    size_t mpatch_cap = 0;
 };
 
 struct MixedState {
     bool ready = false;
+    bool tc_ready = false;           // the tensor-core form's data (element matrices of no modal form)
+    ModalTile mt;                    // modal form: the tile
     float4 *d_bmat = nullptr;        // K_u split [hi, lo][kBFl] in the canonical layout
     std::vector<double> kunif;       // K_u (host), to compare systems of a batch
     Edge edge{};
@@ -1276,15 +1281,9 @@ static int encode_input_map(const Op &op, VecSet &v) {
 static int vecset_alloc(const Op &op, VecSet &v, int part_cap) {
     const size_t n = (size_t)op.ndof;
     int rc;
-    if ((rc = dalloc(&v.patch32, (size_t)op.g.nbricks * 3 * kPVol, "alloc mixed"))) return rc;
-    float **f32[] = {&v.rhs32, &v.x32, &v.r32, &v.p32, &v.ap32, &v.inv32};
+    float **f32[] = {&v.rhs32, &v.x32, &v.r32, &v.p32, &v.inv32};
     for (float **p : f32)
         if ((rc = dalloc(p, n, "alloc mixed"))) return rc;
-    v.cxp = (op.g.cx + 3) & ~3;
-    const size_t npad = (size_t)3 * v.cxp * op.g.cy * op.g.cz;
-    if ((rc = dalloc(&v.pin32, npad, "alloc mixed"))) return rc;
-    ICC_CUDA(cudaMemset(v.pin32, 0, npad * sizeof(float)), "clear apply input");
-    if ((rc = encode_input_map(op, v))) return rc;
     double **f64[] = {&v.x64, &v.r64, &v.y64};
     for (double **p : f64)
         if ((rc = dalloc(p, n, "alloc mixed"))) return rc;
@@ -1293,8 +1292,38 @@ static int vecset_alloc(const Op &op, VecSet &v, int part_cap) {
     return ICC_OK;
 }
 
+// What only one of the two forms needs, allocated on its first use.
+static int vecset_tc(Op &op, VecSet &v) {
+    if (v.pin32) return ICC_OK;
+    int rc;
+    if (!v.ap32 && (rc = dalloc(&v.ap32, (size_t)op.ndof, "alloc mixed"))) return rc;
+    if ((rc = dalloc(&v.patch32, (size_t)op.g.nbricks * 3 * kPVol, "alloc mixed"))) return rc;
+    v.cxp = (op.g.cx + 3) & ~3;
+    const size_t npad = (size_t)3 * v.cxp * op.g.cy * op.g.cz;
+    if ((rc = dalloc(&v.pin32, npad, "alloc mixed"))) return rc;
+    ICC_CUDA(cudaMemsetAsync(v.pin32, 0, npad * sizeof(float), op.stream), "clear apply input");
+    ICC_CUDA(cudaStreamSynchronize(op.stream), "clear apply input");
+    return encode_input_map(op, v);
+}
+static int vecset_modal(Op &op, VecSet &v, const Tiles &t) {
+    int rc;
+    if (!v.p32b && (rc = dalloc(&v.p32b, (size_t)op.ndof, "alloc mixed"))) return rc;
+    if (!v.z32 && (rc = dalloc(&v.z32, (size_t)op.ndof, "alloc mixed"))) return rc;
+    if (op.sp_nnz && !v.ap32 && (rc = dalloc(&v.ap32, (size_t)op.ndof, "alloc mixed"))) return rc;
+    const size_t need = (size_t)t.n * t.vol;
+    if (need > v.mpatch_cap) {
+        if (v.mpatch) cudaFree(v.mpatch);
+        v.mpatch = nullptr;
+        v.mpatch_cap = 0;
+        if ((rc = dalloc(&v.mpatch, need, "alloc mixed"))) return rc;
+        v.mpatch_cap = need;
+    }
+    return ICC_OK;
+}
+
 static void vecset_free(VecSet &v) {
-    void *bufs[] = {v.patch32, v.rhs32, v.x32, v.r32, v.p32, v.ap32, v.inv32, v.pin32, v.x64, v.r64, v.y64, v.part};
+    void *bufs[] = {v.patch32, v.rhs32, v.x32, v.r32, v.p32, v.ap32, v.inv32, v.pin32, v.x64, v.r64, v.y64, v.part,
+                    v.p32b, v.z32, v.mpatch};
     for (void *p : bufs)
         if (p) cudaFree(p);
     v = VecSet();
@@ -1320,14 +1349,10 @@ static void append_descs(const Op &op, int inst, std::vector<BrickDesc> &out) {
     }
 }
 
-static int mixed_init(Op &op) {
-    if (op.mixed && op.mixed->ready) return ICC_OK;
-    if (3LL * ((op.g.cx + 3) & ~3) * op.g.cy * op.g.cz + 4LL * kTailThreads * 1024 >= (1LL << 31))
-        return set_error(ICC_BAD_ARG, "tensor-core path: more than 2^31 DOF");
-    if (op.g.nbx > 2047 || op.g.nby > 2047 || op.g.nbz > 2047)
-        return set_error(ICC_BAD_ARG, "tensor-core path: more than 2047 bricks along a direction");
-    if (!op.mixed) op.mixed = new MixedState();
+// The tensor-core form's own data: the boundary extraction, the split element matrix and the brick list.
+static int mixed_init_tc(Op &op) {
     MixedState &ms = *op.mixed;
+    if (ms.tc_ready) return ICC_OK;
     int rc = setup_edge(op, ms.edge, ms.kunif);
     if (rc) return rc;
     // the uniform element matrix split into TF32 hi/lo in the canonical layout, component c of
@@ -1362,8 +1387,6 @@ static int mixed_init(Op &op) {
             }
         }
         ms.flags = fl;
-        if ((g.nbricks + op.num_sms - 1) / op.num_sms > kMaxListPerCta)
-            return set_error(ICC_BAD_ARG, "tensor-core path: more than 2048 bricks per SM");
         std::vector<BrickDesc> dv;
         append_descs(op, 0, dv);
         if ((rc = dalloc(&ms.d_desc, dv.size(), "alloc brick list"))) return rc;
@@ -1373,6 +1396,26 @@ static int mixed_init(Op &op) {
         ICC_CUDA(cudaMemcpyAsync(ms.d_edge, &ms.edge, sizeof(Edge), cudaMemcpyHostToDevice, op.stream), "copy edge");
         ICC_CUDA(cudaStreamSynchronize(op.stream), "copy brick list");
     }
+    ICC_CUDA(cudaFuncSetAttribute(apply_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem),
+             "cudaFuncSetAttribute tc");
+    ms.tc_ready = true;
+    return ICC_OK;
+}
+
+static int mixed_init(Op &op) {
+    if (op.mixed && op.mixed->ready) return ICC_OK;
+    if (3LL * ((op.g.cx + 3) & ~3) * op.g.cy * op.g.cz + 4LL * kTailThreads * 1024 >= (1LL << 31))
+        return set_error(ICC_BAD_ARG, "tensor-core path: more than 2^31 DOF");
+    if (op.g.nbx > 2047 || op.g.nby > 2047 || op.g.nbz > 2047)
+        return set_error(ICC_BAD_ARG, "tensor-core path: more than 2047 bricks along a direction");
+    if (!op.mixed) op.mixed = new MixedState();
+    MixedState &ms = *op.mixed;
+    int rc;
+    if ((op.g.nbricks + op.num_sms - 1) / op.num_sms > kMaxListPerCta)
+        return set_error(ICC_BAD_ARG, "tensor-core path: more than 2048 bricks per SM");
+    if (op.modal.ok) {
+        ms.mt = modal_tile<float>(op.g, op.num_sms);
+    } else if ((rc = mixed_init_tc(op))) return rc;
     {
         int per_sm = 0;
         ICC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_tail_kernel, kTailThreads, 0),
@@ -1381,6 +1424,7 @@ static int mixed_init(Op &op) {
     }
     if ((rc = dalloc(&ms.d_scale32, (size_t)op.nel, "alloc mixed"))) return rc;
     if ((rc = vecset_alloc(op, ms.v, tail_capacity(op)))) return rc;
+    if ((rc = op.modal.ok ? vecset_modal(op, ms.v, ms.mt.t) : vecset_tc(op, ms.v))) return rc;
     if ((rc = dalloc(&ms.d_scalars, 8, "alloc mixed"))) return rc;
     if ((rc = dalloc(&ms.d_grid_ctr, 1, "alloc mixed"))) return rc;
     if ((rc = dalloc(&ms.d_err, 1, "alloc mixed"))) return rc;
@@ -1392,8 +1436,6 @@ static int mixed_init(Op &op) {
     ICC_CUDA(cudaMemsetAsync(ms.d_err, 0, sizeof(int), op.stream), "clear err");
     ICC_CUDA(cudaMemsetAsync(ms.d_grid_ctr, 0, sizeof(unsigned long long), op.stream), "clear grid counter");
     ICC_CUDA(cudaStreamSynchronize(op.stream), "clear err");
-    ICC_CUDA(cudaFuncSetAttribute(apply_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem),
-             "cudaFuncSetAttribute tc");
     ms.ready = true;
     return mixed_on_scale_update(op);
 }
@@ -1469,6 +1511,30 @@ static TcInst make_inst(const Op &op, const VecSet &v, PcgState *st, int cta0, i
     return I;
 }
 
+// The same for the modal form.
+static ModalSys<float> make_modal(const Op &op, const VecSet &v, const ModalTile &t, PcgState *st,
+                                  unsigned long long *bar, int ncta) {
+    ModalSys<float> S = modal_sys<float>(op, t);
+    S.scale = op.mixed->d_scale32;
+    S.patch = v.mpatch;
+    S.inv = v.inv32;
+    S.r = v.r32;
+    S.z = v.z32;
+    S.p[0] = v.p32;
+    S.p[1] = v.p32b;
+    S.xs = v.x32;
+    S.ap = v.ap32;
+    S.p_zero = op.mask_mode == ICC_MASK_ZERO;
+    S.sp = op.extra32();
+    S.dot = op.sp_nnz == 0;
+    S.part_a = v.part;
+    S.part_v = v.part + ncta;
+    S.bar = bar;
+    S.st = st;
+    S.ncta = ncta;
+    return S;
+}
+
 // The apply may start while the previous kernel of the stream finishes (programmatic dependent
 // launch): it sets up TMEM, its barriers and the B copy, then waits for that kernel.
 static cudaError_t launch_apply_tc(cudaStream_t s, const TcInst *d_insts, int ninst, int nbricks,
@@ -1518,9 +1584,9 @@ static int enqueue_apply_tc(Op &op, const float *x, float *y) {
 
 // Clears the device error flag and the grid-barrier counter before a call, so a handle whose
 // previous call timed out starts clean (stream-ordered before the call's kernels).
-static int clear_flags(cudaStream_t s, int *d_err, unsigned long long *d_ctr) {
+static int clear_flags(cudaStream_t s, int *d_err, unsigned long long *d_ctr, int nctr = 1) {
     ICC_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), s), "clear err");
-    ICC_CUDA(cudaMemsetAsync(d_ctr, 0, sizeof(unsigned long long), s), "clear grid counter");
+    ICC_CUDA(cudaMemsetAsync(d_ctr, 0, (size_t)nctr * sizeof(unsigned long long), s), "clear grid counter");
     return ICC_OK;
 }
 
@@ -1529,11 +1595,27 @@ static int timeout_error(int err) {
                                            : "tensor-core apply: mbarrier wait ran out");
 }
 
-// y32 = A x32 on the tensor cores (icc_op_apply_f32).
+// The modal FP32 contraction of x into the handle's tile partial sums.
+static cudaError_t enqueue_modal(Op &op, const float *x) {
+    MixedState &ms = *op.mixed;
+    ModalSys<float> S = make_modal(op, ms.v, ms.mt, nullptr, nullptr, 0);
+    S.x = x;
+    return launch_modal_apply<float>(op.stream, op.modal, S, ms.mt);
+}
+
+// y32 = A x32 (icc_op_apply_f32).
 int mixed_apply_f32(Op &op, const float *x, float *y) {
     int rc = mixed_init(op);
     if (rc) return rc;
     MixedState &ms = *op.mixed;
+    if (op.modal.ok) {
+        ICC_CUDA(enqueue_modal(op, x), "modal apply launch");
+        gather_kernel<float><<<op.vec_blocks, kVecThreads, 0, op.stream>>>(op.g, ms.mt.t, ms.v.mpatch, x, op.d_mask,
+                                                                           op.mask_mode, op.extra32(), y, nullptr, nullptr);
+        ICC_CUDA(cudaGetLastError(), "modal apply launch");
+        ICC_CUDA(cudaStreamSynchronize(op.stream), "modal apply");
+        return ICC_OK;
+    }
     if ((rc = clear_flags(op.stream, ms.d_err, ms.d_grid_ctr))) return rc;
     if ((rc = enqueue_apply_tc(op, x, y))) return rc;
     ICC_CUDA(cudaMemcpyAsync(ms.h_err, ms.d_err, sizeof(int), cudaMemcpyDeviceToHost, op.stream), "err");
@@ -1564,19 +1646,25 @@ int mixed_profile_apply(Op &op, const float *x, float *y, int reps, double *cont
     if (rc) return rc;
     MixedState &ms = *op.mixed;
     if ((rc = clear_flags(op.stream, ms.d_err, ms.d_grid_ctr))) return rc;
-    enqueue_pad_input(op, ms.v, x, op.stream);
-    const TcInst I = make_inst(op, ms.v, nullptr, 0, 0, 1.f);
-    ICC_CUDA(cudaMemcpyAsync(ms.d_inst, &I, sizeof(TcInst), cudaMemcpyHostToDevice, op.stream), "instance table");
+    const bool modal = op.modal.ok;
+    if (!modal) {
+        enqueue_pad_input(op, ms.v, x, op.stream);
+        const TcInst I = make_inst(op, ms.v, nullptr, 0, 0, 1.f);
+        ICC_CUDA(cudaMemcpyAsync(ms.d_inst, &I, sizeof(TcInst), cudaMemcpyHostToDevice, op.stream), "instance table");
+    }
+    const Tiles t = modal ? ms.mt.t : brick_tiles(op.g);
+    const float *patch = modal ? ms.v.mpatch : ms.v.patch32;
     std::vector<cudaEvent_t> ev(3 * size_t(reps));
     for (auto &e : ev) ICC_CUDA(cudaEventCreate(&e), "event create");
     for (int r = 0; r < reps; ++r) {
         cudaEventRecord(ev[3 * r], op.stream);
-        ICC_CUDA(launch_apply_tc(op.stream, ms.d_inst, 1, op.g.nbricks, ms.d_desc, ms.d_bmat, ms.d_err, op.num_sms),
-                 "tc apply launch");
+        if (modal) ICC_CUDA(enqueue_modal(op, x), "modal apply launch");
+        else
+            ICC_CUDA(launch_apply_tc(op.stream, ms.d_inst, 1, op.g.nbricks, ms.d_desc, ms.d_bmat, ms.d_err, op.num_sms),
+                     "tc apply launch");
         cudaEventRecord(ev[3 * r + 1], op.stream);
-        gather_kernel<float><<<op.vec_blocks, kVecThreads, 0, op.stream>>>(op.g, brick_tiles(op.g), ms.v.patch32, x, op.d_mask,
-                                                                           ICC_MASK_NONE, op.extra32(), y, nullptr,
-                                                                           nullptr);
+        gather_kernel<float><<<op.vec_blocks, kVecThreads, 0, op.stream>>>(op.g, t, patch, x, op.d_mask, ICC_MASK_NONE,
+                                                                           op.extra32(), y, nullptr, nullptr);
         cudaEventRecord(ev[3 * r + 2], op.stream);
     }
     cudaError_t e = cudaEventSynchronize(ev.back());
@@ -1609,12 +1697,14 @@ __global__ void ru_accumulate_kernel(long long n, double *__restrict__ x, float 
 // r32 = r64 / sigma (the FP64 residual replaces the FP32 recurrence residual); partials r'z, r'r
 __global__ void __launch_bounds__(kVecThreads)
 ru_replace_kernel(long long n, const double *__restrict__ r64, double inv_sigma, const float *__restrict__ inv,
-                  float *__restrict__ r32, double *__restrict__ partials) {
+                  float *__restrict__ r32, float *__restrict__ z32, double *__restrict__ partials) {
     double rz = 0.0, rr = 0.0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         float ri = float(r64[i] * inv_sigma);
+        const float zi = inv[i] * ri;
         r32[i] = ri;
-        rz += double(ri) * double(inv[i] * ri);
+        if (z32) z32[i] = zi;
+        rz += double(ri) * double(zi);
         rr += double(ri) * double(ri);
     }
     rz = block_sum(rz);
@@ -1681,6 +1771,8 @@ struct MixedBatch {
     int ninst = 0, nbricks = 0, tail_grid = 0, num_sms = 148;
     const float4 *bmat = nullptr;
     long long limit = kGridWaitLimit;
+    Op *modal = nullptr;   // one system whose operator has the modal form
+    ModalSys<float> sys{};
     bool owned = false;   // allocated for this call (a batch), else borrowed from the handle
     ~MixedBatch() {
         if (!owned) return;
@@ -1730,7 +1822,7 @@ static int init_items(MixedBatch &bt, std::vector<MixedItem> &items, double delt
     cudaStream_t s = bt.stream;
     const size_t m = items.size();
     int rc;
-    if ((rc = clear_flags(s, bt.d_err, bt.d_ctr))) return rc;
+    if ((rc = clear_flags(s, bt.d_err, bt.d_ctr, bt.ninst))) return rc;
     for (size_t i = 0; i < m; ++i) {
         MixedItem &it = items[i];
         Op &op = *it.op;
@@ -1766,15 +1858,32 @@ static int init_items(MixedBatch &bt, std::vector<MixedItem> &items, double delt
         const uint8_t *pm = op.mask_mode == ICC_MASK_ZERO ? op.d_mask : nullptr;
         ir_to_f32_kernel<<<op.vec_blocks, kVecThreads, 0, s>>>(op.ndof, v.r64, v.rhs32, bt.d_scalars + i);
         pcg_init_kernel<float><<<op.vec_blocks, kVecThreads, 0, s>>>(op.ndof, v.rhs32, v.inv32, v.x32, v.r32, v.p32,
-                                                                     op.d_partials, pm);
+                                                                     op.d_partials, pm, bt.modal ? v.z32 : nullptr);
         pcg_init_finalize<<<1, kVecThreads, 0, s>>>(op.d_partials, op.vec_blocks, bt.d_state + i, trial ? 0.0 : it.tol,
                                                     trial ? (1LL << 40) : (long long)it.max_iter);
         ru_arm_kernel<<<1, 1, 0, s>>>(bt.d_state + i, 1.0, trial ? 0.0 : delta, kMaxSegment, check_every);
         launches += 4;
-        enqueue_pad_input(op, v, v.p32, s);
-        launches++;
+        if (!bt.modal) {
+            enqueue_pad_input(op, v, v.p32, s);
+            launches++;
+        }
     }
     ICC_CUDA(cudaGetLastError(), "mixed init");
+    return ICC_OK;
+}
+
+static int nan_error(const MixedItem &it, const PcgState &hs) {
+    return set_error(ICC_NAN, "mixed solve: non-finite residual (FP64 " + std::to_string(it.res) + ", FP32 " +
+                                  std::to_string(hs.rel_res) + ", p'Ap " + std::to_string(hs.p_ap) + ", iteration " +
+                                  std::to_string(hs.iter) + ", update " + std::to_string(it.updates) + ")");
+}
+
+// The one system of a batch in the modal form.
+static int set_modal(MixedBatch &bt, Op &op, VecSet &v) {
+    int rc;
+    if ((rc = vecset_modal(op, v, op.mixed->mt.t))) return rc;
+    bt.modal = &op;
+    bt.sys = make_modal(op, v, op.mixed->mt, bt.d_state, bt.d_ctr, modal_ctas(op.g, op.mixed->mt, op.num_sms));
     return ICC_OK;
 }
 
@@ -1793,14 +1902,19 @@ static int run_mixed(MixedBatch &bt, std::vector<MixedItem> &items, const icc_so
     int rc;
     if ((rc = init_items(bt, items, delta, check_every, false, launches))) return rc;
 
+    // the modal form leaves its launch by itself when it wants a replacement or stops
+    const int batch = bt.modal ? 8 * check_every : check_every;
     int64_t launched = 0, max_budget = 0;
     for (const auto &it : items) max_budget = std::max(max_budget, it.max_iter);
     size_t active = 0;
     for (const auto &it : items) active += it.done ? 0 : 1;
     while (active > 0) {
-        ICC_CUDA(cudaGraphLaunch(bt.graph, s), "graph launch");
-        launches += 2 * int64_t(check_every);
-        launched += check_every;
+        if (bt.modal)
+            ICC_CUDA(launch_modal_pcg<float>(s, bt.modal->modal, bt.sys, bt.modal->mixed->mt, batch, bt.d_err, bt.limit),
+                     "solve launch");
+        else ICC_CUDA(cudaGraphLaunch(bt.graph, s), "graph launch");
+        launches += bt.modal ? 1 : 2 * int64_t(check_every);
+        launched += batch;
         ICC_CUDA(cudaMemcpyAsync(bt.h_state, bt.d_state, m * sizeof(PcgState), cudaMemcpyDeviceToHost, s), "state");
         ICC_CUDA(cudaMemcpyAsync(bt.h_err, bt.d_err, sizeof(int), cudaMemcpyDeviceToHost, s), "err");
         ICC_CUDA(cudaStreamSynchronize(s), "inner sync");
@@ -1810,7 +1924,7 @@ static int run_mixed(MixedBatch &bt, std::vector<MixedItem> &items, const icc_so
         for (size_t i = 0; i < m; ++i)
             if (!items[i].done && bt.h_state[i].status != 0) upd.push_back(i);
         if (upd.empty()) {
-            if (launched > max_budget + 2 * int64_t(check_every))
+            if (launched > max_budget + 2 * int64_t(batch))
                 return set_error(ICC_TIMEOUT, "mixed solve: device state did not reach a stop condition");
             continue;
         }
@@ -1838,10 +1952,7 @@ static int run_mixed(MixedBatch &bt, std::vector<MixedItem> &items, const icc_so
             if (it.res < it.tol) {
                 it.status = ICC_OK;
             } else if (!std::isfinite(it.res) || hs.status == kStatNan) {
-                it.status = set_error(ICC_NAN, "mixed solve: non-finite residual (FP64 " + std::to_string(it.res) +
-                                                   ", FP32 " + std::to_string(hs.rel_res) + ", p'Ap " +
-                                                   std::to_string(hs.p_ap) + ", iteration " + std::to_string(hs.iter) +
-                                                   ", update " + std::to_string(it.updates) + ")");
+                it.status = nan_error(it, hs);
             } else if (hs.status == kStatBreakdown) {
                 it.status = ICC_BREAKDOWN;
             } else if (hs.status == kStatMaxIter || hs.iter >= it.max_iter || it.updates >= max_updates) {
@@ -1861,15 +1972,17 @@ static int run_mixed(MixedBatch &bt, std::vector<MixedItem> &items, const icc_so
                 active--;
                 continue;
             }
-            ru_replace_kernel<<<op.vec_blocks, kVecThreads, 0, s>>>(op.ndof, v.r64, 1.0 / it.nb, v.inv32, v.r32,
+            ru_replace_kernel<<<op.vec_blocks, kVecThreads, 0, s>>>(op.ndof, v.r64, 1.0 / it.nb, v.inv32, v.r32, bt.modal ? v.z32 : nullptr,
                                                                     op.d_partials);
             ru_replace_finalize<<<1, kVecThreads, 0, s>>>(op.d_partials, op.vec_blocks, bt.d_state + i);
             ru_arm_kernel<<<1, 1, 0, s>>>(bt.d_state + i, it.res, delta, kMaxSegment, check_every);
+            launches += 3;
+            if (bt.modal) continue;   // the next apply forms the direction
             // the direction update of this iteration, with the replaced residual
             pcg_p_kernel<float><<<op.vec_blocks, kVecThreads, 0, s>>>(op.ndof, v.r32, v.inv32, v.p32, bt.d_state + i,
                                                                       op.mask_mode == ICC_MASK_ZERO ? op.d_mask : nullptr);
             enqueue_pad_input(op, v, v.p32, s);
-            launches += 5;
+            launches += 2;
         }
         ICC_CUDA(cudaGetLastError(), "replacement");
     }
@@ -1939,8 +2052,9 @@ int mixed_solve(Op &op, const double *b, const double *diag, double tol, int64_t
     bt.num_sms = op.num_sms;
     bt.bmat = ms.d_bmat;
     bt.limit = ms.grid_wait_limit;
-    bt.graph = ms.graph;
-    if (!ms.graph || ms.graph_batch != check_every || ms.graph_limit != ms.grid_wait_limit) {
+    if (op.modal.ok) {
+        if ((rc = set_modal(bt, op, ms.v))) return rc;
+    } else if (!ms.graph || ms.graph_batch != check_every || ms.graph_limit != ms.grid_wait_limit) {
         const TcInst I = make_inst(op, ms.v, ms.d_state, 0, bt.tail_grid, 1.f);
         ICC_CUDA(cudaMemcpyAsync(bt.d_inst, &I, sizeof(TcInst), cudaMemcpyHostToDevice, op.stream), "instance table");
         bt.graph = ms.graph;
@@ -2053,10 +2167,14 @@ static int autotune(MixedBatch &bt, std::vector<MixedItem> &items, int max_per_s
             if ((rc = upload_table(bt, items, ncta)) || (rc = capture_graph(bt, kTuneIters)) ||
                 (rc = init_items(bt, items, 0.0, kTuneIters, true, l)))
                 break;
-            cudaGraphLaunch(bt.graph, bt.stream);
+            cudaError_t ge = cudaGraphLaunch(bt.graph, bt.stream);
             cudaEventRecord(e0, bt.stream);
-            cudaGraphLaunch(bt.graph, bt.stream);
+            if (ge == cudaSuccess) ge = cudaGraphLaunch(bt.graph, bt.stream);
             cudaEventRecord(e1, bt.stream);
+            if (ge != cudaSuccess) {
+                rc = cuda_fail(ge, "autotune");
+                break;
+            }
             cudaError_t e = cudaEventSynchronize(e1);
             if (e != cudaSuccess) {
                 rc = cuda_fail(e, "autotune");
@@ -2097,12 +2215,18 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
         ICC_CUDA(cudaStreamSynchronize(op->stream), "batch: drain handle");
     }
     // every system's K_u must be the first one's times a factor (elements of one shape)
-    const std::vector<double> &K0 = ops[0]->mixed->kunif;
+    bool modal = m == 1;
+    for (Op *op : ops) modal = modal && op->modal.ok;
+    if (!modal)
+        for (size_t i = 0; i < m; ++i)
+            if ((rc = mixed_init_tc(*ops[i])) || (rc = vecset_tc(*ops[i], *vsets[i]))) return rc;
+    auto kunif = [&](size_t i) -> const std::vector<double> & { return modal ? ops[i]->modal.kunif : ops[i]->mixed->kunif; };
+    const std::vector<double> &K0 = kunif(0);
     double k0max = 0.0;
     for (double v : K0) k0max = std::fmax(k0max, std::fabs(v));
     std::vector<float> kfac(m, 1.f);
     for (size_t i = 0; i < m; ++i) {
-        const std::vector<double> &Ki = ops[i]->mixed->kunif;
+        const std::vector<double> &Ki = kunif(i);
         double num = 0.0, den = 0.0;
         for (size_t k = 0; k < Ki.size(); ++k) {
             num += Ki[k] * K0[k];
@@ -2128,7 +2252,7 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
         items[i].max_iter = max_iter[i];
         items[i].x_out = x[i];
         items[i].kfac = kfac[i];
-        append_descs(*ops[i], (int)i, descs);
+        if (!modal) append_descs(*ops[i], (int)i, descs);
         nbricks += ops[i]->g.nbricks;
     }
     if ((nbricks + ops[0]->num_sms - 1) / ops[0]->num_sms > kMaxListPerCta)
@@ -2147,13 +2271,14 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
     if ((rc = dalloc(&bt.d_inst, m, "alloc batch")) || (rc = dalloc(&bt.d_desc, descs.size(), "alloc batch")) ||
         (rc = dalloc(&bt.d_state, m, "alloc batch")) ||
         (rc = dalloc(&bt.d_scalars, m, "alloc batch")) || (rc = dalloc(&bt.d_err, 1, "alloc batch")) ||
-        (rc = dalloc(&bt.d_ctr, 1, "alloc batch")))
+        (rc = dalloc(&bt.d_ctr, m, "alloc batch")))
         return rc;
     ICC_CUDA(cudaMallocHost((void **)&bt.h_state, m * sizeof(PcgState)), "alloc pinned");
     ICC_CUDA(cudaMallocHost((void **)&bt.h_scalars, m * sizeof(double)), "alloc pinned");
     ICC_CUDA(cudaMallocHost((void **)&bt.h_err, sizeof(int)), "alloc pinned");
-    ICC_CUDA(cudaMemcpyAsync(bt.d_desc, descs.data(), descs.size() * sizeof(BrickDesc), cudaMemcpyHostToDevice, stream),
-             "brick list");
+    if (!descs.empty())
+        ICC_CUDA(cudaMemcpyAsync(bt.d_desc, descs.data(), descs.size() * sizeof(BrickDesc), cudaMemcpyHostToDevice, stream),
+                 "brick list");
     // the vector step's CTAs: tuned once per batch shape (a single system takes them all)
     TuneChoice ch;
     ch.per_sm = ops[0]->mixed->tail_per_sm;
@@ -2176,9 +2301,12 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
             tune_save();
         }
     }
-    if ((rc = upload_table(bt, items, share_ctas(items, ch.per_sm * bt.num_sms, ch.share)))) return rc;
-    const int check_every = opts.check_every > 0 ? opts.check_every : 32;
-    if ((rc = capture_graph(bt, check_every))) return rc;
+    if (modal) {
+        if ((rc = set_modal(bt, *ops[0], *vsets[0]))) return rc;
+    } else {
+        if ((rc = upload_table(bt, items, share_ctas(items, ch.per_sm * bt.num_sms, ch.share)))) return rc;
+        if ((rc = capture_graph(bt, opts.check_every > 0 ? opts.check_every : 32))) return rc;
+    }
     rc = run_mixed(bt, items, opts, nullptr);
     if (rc) return rc;
     for (size_t i = 0; i < m; ++i) {

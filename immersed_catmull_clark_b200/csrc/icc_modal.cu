@@ -173,48 +173,62 @@ bool modal_setup(const Op &op, ModalHost &m) {
 
 // ---- the tile ------------------------------------------------------------------------------------
 
-// Columns of a tile (threads), its extent and length, by a model of the launch: clocks of a CTA's march
-// (per warp and step, for planes and for elements, measured with the kernel alone on the chip) times the
-// waves of CTAs.  Short marches of small tiles fill the chip on small grids, where latency counts;
-// 256 columns waste the least on the two extra planes of a tile and on its overlap.
+// Cubes or a march, and its tile, by a model of the kernel in clocks (all measured with the kernels alone on the
+// chip): a cube takes its share of an SM's pipes or its own latency, a march its steps (of elements and
+// of planes alone) in rounds of one per SM; fewer columns make shorter steps.  Measured, us an iteration of
+// solves forced to cubes / marches of 128 / 256 / 512 columns: FP32 12.4 / 21.1 / 23.0 at 24x16x12, 24.0 / 24.9 /
+// 23.9 at 53x31x27, 148.9 / 114.8 / 77.8 / 69.8 at 128x64x64; FP64 12.6 / 22.3 / 26.1, 27.3 / 27.0 / 27.2 and
+// 214 / 148 / 105 there.
 template <class T>
-ModalTile modal_tile(const Geom &g, int num_sms) {
+static void modal_plan(const Geom &g, int sms, ModalTile &best) {
     const bool f64 = sizeof(T) == 8;
-    const double c_el = f64 ? 1500.0 : 700.0, c_pl = f64 ? 700.0 : 400.0, c_step = 500.0, c_start = 2500.0;
-    ModalTile best;
-    double cost = INFINITY;
-    struct Shape { int nt, ltx, per_sm; };
-    // FP64: 256 columns' state fills tensor memory; FP32: 512
-    const Shape f64_shapes[] = {{256, 5, 1}, {256, 4, 1}, {64, 4, 2}, {64, 3, 2}};
-    const Shape f32_shapes[] = {{512, 5, 1}, {512, 4, 1}, {64, 4, 4}, {64, 3, 4}};
-    const Shape (&shapes)[4] = f64 ? f64_shapes : f32_shapes;
-    for (const Shape &s : shapes) {
-        const int tx = 1 << s.ltx, rows = s.nt >> s.ltx;
-        if (tx > 8 && tx >= 2 * g.nx) continue;
-        for (int nty = (g.ny + rows - 1) / rows, k = 0; k < 3; ++k, ++nty) {
-            const int ty = (g.ny + nty - 1) / nty;
-            if (ty < 2 && g.ny > 1) break;
-            for (int ntz = 1; ntz <= g.nz; ++ntz) {
-                const int tz = (g.nz + ntz - 1) / ntz;
-                if (tz < 2 && g.nz > 1) break;
-                const long long n = (long long)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty) * ((g.nz + tz - 1) / tz);
-                const long long slots = (long long)num_sms * s.per_sm, waves = (n + slots - 1) / slots;
-                const long long on_sm = std::min<long long>(s.per_sm, (n + num_sms - 1) / num_sms);
-                const double warps = std::max(1.0, (double)on_sm * s.nt / 128.0);   // per scheduler
-                const double march = warps * (tz * c_el + (tz + 2) * c_pl) + (tz + 5) * c_step;
-                const double c = waves * march + c_start;
-                if (c < cost) {
-                    cost = c;
-                    best.nt = s.nt;
-                    best.t = make_tiles(g.nx, g.ny, g.nz, tx, ty, tz);
+    const Tiles cubes = make_tiles(g.nx, g.ny, g.nz, kCube, kCube, kCube);
+    double cost = std::fmax(f64 ? 7500.0 : 6700.0, (double)cubes.n / sms * (f64 ? 7000.0 : 4800.0));
+    best.nt = 0;
+    best.t = cubes;
+    // clocks of an element step and of a plane-only step by columns
+    struct Step { int nt; double el, pl; };
+    const Step f64_steps[] = {{128, 5400.0, 2400.0}, {256, 7000.0, 3100.0}};
+    const Step f32_steps[] = {{128, 4850.0, 2150.0}, {256, 5800.0, 2500.0}, {512, 9200.0, 4100.0}};
+    const Step *st = f64 ? f64_steps : f32_steps;
+    for (int q = 0; q < (f64 ? 2 : 3); ++q) {
+        for (int ltx = 5; ltx >= 4; --ltx) {
+            const int tx = 1 << ltx, rows = st[q].nt >> ltx;
+            if (tx == 32 && tx >= 2 * g.nx) continue;
+            for (int nty = (g.ny + rows - 1) / rows, k = 0; k < 3; ++k, ++nty) {
+                const int ty = (g.ny + nty - 1) / nty;
+                if (ty < 2 && g.ny > 1) break;
+                for (int ntz = 1; ntz <= g.nz; ++ntz) {
+                    const int tz = (g.nz + ntz - 1) / ntz;
+                    if (tz < 2 && g.nz > 1) break;
+                    const double n = (double)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty) * ((g.nz + tz - 1) / tz);
+                    if (n > 1e9) break;
+                    const double c = std::ceil(n / sms) * (tz * st[q].el + 5 * st[q].pl);
+                    if (c < cost) {
+                        cost = c;
+                        best.nt = st[q].nt;
+                        best.t = make_tiles(g.nx, g.ny, g.nz, tx, ty, tz);
+                    }
                 }
             }
         }
     }
-    return best;
+}
+
+// Of a plain apply (a CTA a tile) and of a solve (tiles dealt to a CTA per SM).
+template <class T>
+ModalTile modal_tile(const Geom &g, int num_sms) {
+    ModalTile t;
+    modal_plan<T>(g, num_sms, t);
+    return t;
 }
 template ModalTile modal_tile<double>(const Geom &g, int num_sms);
 template ModalTile modal_tile<float>(const Geom &g, int num_sms);
+
+// CTAs of a solve of one system: no more than it has tiles or control points for.
+int modal_ctas(const Geom &g, const ModalTile &t, int num_sms) {
+    return std::min(num_sms, std::max(t.t.n, (int)((g.nsc + 511) / 512)));
+}
 
 // ---- launches -------------------------------------------------------------------------------------
 
@@ -229,37 +243,69 @@ ModalK<T> modal_entries(const ModalHost &m) {
                 for (int l = 0; l < 3; ++l) k.off[p][q][n][l] = T(m.off[p][q][n][l]);
     return k;
 }
-template ModalK<double> modal_entries<double>(const ModalHost &m);
-template ModalK<float> modal_entries<float>(const ModalHost &m);
 
-template <class T, int NT, bool PCG, bool MANY>
-static cudaError_t launch_one(cudaStream_t s, const ModalK<T> &K, const ModalSys<T> &one, const ModalSys<T> *many,
-                              const int2 *list, int ntiles, int ltx) {
-    const size_t smem = modal_smem<T>(NT, ltx, ModalCfg<T, NT>::slots, PCG);
-    const cudaError_t e = cudaFuncSetAttribute(modal_apply_kernel<T, NT, PCG, MANY>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+constexpr int kMaxDynSmem = 224 * 1024;   // beside the kernels' static 1.7 KB
+
+template <class T, int NT>
+static cudaError_t launch_march(cudaStream_t s, const ModalK<T> &K, const ModalSys<T> &S, const ModalTile &t) {
+    const cudaError_t e = cudaFuncSetAttribute(modal_march_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
     if (e != cudaSuccess) return e;
-    modal_apply_kernel<T, NT, PCG, MANY><<<ntiles, NT, smem, s>>>(K, one, many, list);
+    modal_march_kernel<T, NT><<<t.t.n, NT, march_smem(NT, t.t.ltx, false) * sizeof(T), s>>>(K, S);
     return cudaGetLastError();
 }
 
 template <class T>
-cudaError_t launch_modal_apply(cudaStream_t s, const ModalK<T> &K, const ModalSys<T> &one, const ModalSys<T> *many,
-                               const int2 *list, int ntiles, int nt, int ltx, bool pcg) {
-    constexpr int kWide = sizeof(T) == 8 ? 256 : 512;
-    if (nt == kWide) {
-        if (many) return launch_one<T, kWide, true, true>(s, K, one, many, list, ntiles, ltx);
-        return pcg ? launch_one<T, kWide, true, false>(s, K, one, many, list, ntiles, ltx)
-                   : launch_one<T, kWide, false, false>(s, K, one, many, list, ntiles, ltx);
+cudaError_t launch_modal_apply(cudaStream_t s, const ModalHost &m, const ModalSys<T> &S, const ModalTile &t) {
+    const ModalK<T> K = modal_entries<T>(m);
+    if (t.nt == 0) {
+        const cudaError_t e = cudaFuncSetAttribute(modal_cube_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+        if (e != cudaSuccess) return e;
+        modal_cube_kernel<T><<<t.t.n, kCubeThreads, kCubeSmem * sizeof(T), s>>>(K, S);
+        return cudaGetLastError();
     }
-    if (many) return launch_one<T, 64, true, true>(s, K, one, many, list, ntiles, ltx);
-    return pcg ? launch_one<T, 64, true, false>(s, K, one, many, list, ntiles, ltx)
-               : launch_one<T, 64, false, false>(s, K, one, many, list, ntiles, ltx);
+    if (t.nt == 128) return launch_march<T, 128>(s, K, S, t);
+    if (t.nt == 256) return launch_march<T, 256>(s, K, S, t);
+    if constexpr (sizeof(T) == 4) return launch_march<T, 512>(s, K, S, t);
+    return cudaErrorInvalidValue;
 }
-template cudaError_t launch_modal_apply<double>(cudaStream_t, const ModalK<double> &, const ModalSys<double> &,
-                                                const ModalSys<double> *, const int2 *, int, int, int, bool);
-template cudaError_t launch_modal_apply<float>(cudaStream_t, const ModalK<float> &, const ModalSys<float> &,
-                                               const ModalSys<float> *, const int2 *, int, int, int, bool);
+template cudaError_t launch_modal_apply<double>(cudaStream_t, const ModalHost &, const ModalSys<double> &, const ModalTile &);
+template cudaError_t launch_modal_apply<float>(cudaStream_t, const ModalHost &, const ModalSys<float> &, const ModalTile &);
+
+// Every CTA takes more than half of an SM's shared memory, so two of these kernels (two solves on two
+// streams) never share an SM: tensor memory is then always there for a resident CTA, and no CTA waits
+// for it while others wait for that CTA at a barrier.
+template <class T, int NT>
+static cudaError_t launch_pcg(cudaStream_t s, const ModalHost &m, const ModalSys<T> &S, const ModalTile &t, int iters, int *err,
+                              long long limit) {
+    const int values = NT == 0 ? modal_threads<T, NT>() / kCubeThreads * kCubeSmem : march_smem(NT, t.t.ltx, true);
+    cudaError_t e = cudaFuncSetAttribute(modal_pcg_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)S.ncta);
+    cfg.blockDim = dim3(modal_threads<T, NT>());
+    cfg.dynamicSmemBytes = std::max((size_t)values * sizeof(T), (size_t)120 * 1024);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;   // the barriers need every CTA resident
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, modal_pcg_kernel<T, NT>, modal_entries<T>(m), S, iters, err, limit);
+}
+
+template <class T>
+cudaError_t launch_modal_pcg(cudaStream_t s, const ModalHost &m, const ModalSys<T> &S, const ModalTile &t, int iters, int *err,
+                             long long limit) {
+    if (t.nt == 0) return launch_pcg<T, 0>(s, m, S, t, iters, err, limit);
+    if (t.nt == 128) return launch_pcg<T, 128>(s, m, S, t, iters, err, limit);
+    if (t.nt == 256) return launch_pcg<T, 256>(s, m, S, t, iters, err, limit);
+    if constexpr (sizeof(T) == 4) return launch_pcg<T, 512>(s, m, S, t, iters, err, limit);
+    return cudaErrorInvalidValue;
+}
+template cudaError_t launch_modal_pcg<double>(cudaStream_t, const ModalHost &, const ModalSys<double> &, const ModalTile &, int,
+                                              int *, long long);
+template cudaError_t launch_modal_pcg<float>(cudaStream_t, const ModalHost &, const ModalSys<float> &, const ModalTile &, int,
+                                             int *, long long);
 
 // The grid part of a system's entry.
 template <class T>
@@ -275,7 +321,6 @@ ModalSys<T> modal_sys(const Op &op, const ModalTile &t) {
         S.a[d] = T(op.modal.a[d]);
         S.b[d] = T(op.modal.b[d]);
     }
-    S.kfac = T(1);
     S.mask = op.d_mask;
     S.mask_mode = op.mask_mode;
     return S;

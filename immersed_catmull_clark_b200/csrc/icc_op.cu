@@ -223,6 +223,7 @@ pcg_init_finalize(const double *__restrict__ partials, int np, PcgState *st, dou
         st->repl_iter = 0;
         st->repl_seg = 0;
         st->repl_every = 1;
+        st->bars = 0;
     }
 }
 
@@ -241,11 +242,12 @@ static int dev_alloc(T **p, size_t count, const char *what) {
 Op::~Op() {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     void *bufs[] = {d_x_in, d_y_out, d_scale, d_kfrag, d_kdiag, d_type_id, d_tile_start, d_tile_type, d_tile_elem,
-                    d_mask, d_patch, d_x, d_r, d_p, d_ap, d_inv, d_b, d_diag, d_partials, d_state, d_counter,
+                    d_mask, d_patch, d_x, d_r, d_p, d_p2, d_z, d_part_a, d_bar, d_err, d_ap, d_inv, d_b, d_diag, d_partials, d_state, d_counter,
                     d_sp_ptr, d_sp_idx, d_sp_val, d_sp_val32, d_sp_diag};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (h_state) cudaFreeHost(h_state);
+    if (h_err) cudaFreeHost(h_err);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (stream) cudaStreamDestroy(stream);
@@ -258,10 +260,10 @@ int Op::init(const Space &s, const double *ke_types, int nt, const int32_t *type
     if (cudaGetDevice(&device) != cudaSuccess) return set_error(ICC_NO_DEVICE, "no CUDA device");
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return set_error(ICC_NO_DEVICE, "no CUDA device");
-    cudaDeviceProp prop;
-    ICC_CUDA(cudaGetDeviceProperties(&prop, device), "cudaGetDeviceProperties");
-    if (prop.major < 10) return set_error(ICC_NO_DEVICE, "device is not sm_100 class (B200 required)");
-    num_sms = prop.multiProcessorCount;
+    int major = 0;
+    ICC_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device), "device attributes");
+    if (major < 10) return set_error(ICC_NO_DEVICE, "device is not sm_100 class (B200 required)");
+    ICC_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device), "device attributes");
 
     g.nx = int(s.nel_dir[0]); g.ny = int(s.nel_dir[1]); g.nz = int(s.nel_dir[2]);
     g.cx = int(s.ncp[0]); g.cy = int(s.ncp[1]); g.cz = int(s.ncp[2]);
@@ -306,7 +308,7 @@ int Op::init(const Space &s, const double *ke_types, int nt, const int32_t *type
 
     if ((rc = dev_alloc(&d_scale, (size_t)nel, "alloc scale"))) return rc;
     if ((rc = dev_alloc(&d_mask, (size_t)ndof, "alloc mask"))) return rc;
-    if ((rc = dev_alloc(&d_patch, (size_t)tiles.n * tiles.vol, "alloc patch scratch"))) return rc;
+    if ((rc = dev_alloc(&d_patch, std::max((size_t)tiles.n * tiles.vol, (size_t)mtile.t.n * mtile.t.vol), "alloc patch scratch"))) return rc;
     if ((rc = dev_alloc(&d_x_in, (size_t)ndof, "alloc io"))) return rc;
     if ((rc = dev_alloc(&d_y_out, (size_t)ndof, "alloc io"))) return rc;
     vec_blocks = num_sms * 4;
@@ -501,9 +503,7 @@ cudaError_t Op::enqueue_contract(cudaStream_t s, const double *x, const PcgState
         S.scale = d_scale;
         S.x = x;
         S.patch = d_patch;
-        S.st = const_cast<PcgState *>(st);
-        return launch_modal_apply<double>(s, modal_entries<double>(modal), S, nullptr, nullptr, tiles.n, mtile.nt,
-                                          tiles.ltx, false);
+        return launch_modal_apply<double>(s, modal, S, mtile);
     }
     apply_f64_kernel<<<g.nbricks, kApplyThreads, kApplySmem, s>>>(g, x, d_mask, mask_mode != ICC_MASK_NONE, d_scale,
                                                                    d_kfrag, d_tile_start, d_tile_type, d_tile_elem,
@@ -548,24 +548,53 @@ int Op::ensure_pcg_buffers() {
     if ((rc = dev_alloc(&d_r, (size_t)ndof, "alloc pcg"))) return rc;
     if ((rc = dev_alloc(&d_p, (size_t)ndof, "alloc pcg"))) return rc;
     if ((rc = dev_alloc(&d_ap, (size_t)ndof, "alloc pcg"))) return rc;
+    if (modal.ok) {
+        if ((rc = dev_alloc(&d_p2, (size_t)ndof, "alloc pcg"))) return rc;
+        if ((rc = dev_alloc(&d_z, (size_t)ndof, "alloc pcg"))) return rc;
+        if ((rc = dev_alloc(&d_part_a, (size_t)num_sms, "alloc pcg"))) return rc;
+        if ((rc = dev_alloc(&d_bar, 1, "alloc pcg"))) return rc;
+        if ((rc = dev_alloc(&d_err, 1, "alloc pcg"))) return rc;
+        ICC_CUDA(cudaMallocHost((void **)&h_err, sizeof(int)), "alloc pinned");
+    }
     if ((rc = dev_alloc(&d_inv, (size_t)ndof, "alloc pcg"))) return rc;
     if ((rc = dev_alloc(&d_b, (size_t)ndof, "alloc pcg"))) return rc;
     if ((rc = dev_alloc(&d_diag, (size_t)ndof, "alloc pcg"))) return rc;
     return ICC_OK;
 }
 
-// One PCG iteration (rust/src/solver.rs:40-72) as six launches: p = z + beta p (beta = 0 on the
-// first iteration, so p = z), Ap, alpha, x/r update, convergence test and the next beta.  Every
-// kernel returns at once when the state says the solve has finished, so a batch may overrun
+// One PCG iteration (rust/src/solver.rs:40-72) of the dense form as four launches: p = z + beta p (beta = 0
+// on the first iteration, so p = z), Ap, alpha, x/r update, convergence test and the next beta.
+// Every kernel returns at once when the state says the solve has finished, so a batch may overrun
 // harmlessly.
 void Op::enqueue_pcg_iteration() {
     pcg_p_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(ndof, d_r, d_inv, d_p, d_state);
     enqueue_contract(stream, d_p, d_state);
-    gather_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(g, tiles, d_patch, d_p, d_mask, mask_mode, extra64(), d_ap,
-                                                                  d_partials,
-                                                                  d_state, d_state, d_counter);
+    gather_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(g, tiles, d_patch, d_p, d_mask, mask_mode, extra64(),
+                                                                  d_ap, d_partials, d_state, d_state, d_counter);
     pcg_update_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(ndof, d_p, d_ap, d_inv, d_x, d_r, d_partials,
                                                                       d_state, d_state, d_counter);
+}
+
+// Iterations of the modal form in one launch, up to `iters` or until the solve stops.
+cudaError_t Op::enqueue_pcg_modal(int iters) {
+    ModalSys<double> S = modal_sys<double>(*this, mtile);
+    S.scale = d_scale;
+    S.patch = d_patch;
+    S.inv = d_inv;
+    S.r = d_r;
+    S.z = d_z;
+    S.p[0] = d_p;
+    S.p[1] = d_p2;
+    S.xs = d_x;
+    S.ap = d_ap;
+    S.sp = extra64();
+    S.dot = sp_nnz == 0;
+    S.part_a = d_part_a;
+    S.part_v = d_partials;
+    S.bar = d_bar;
+    S.st = d_state;
+    S.ncta = modal_ctas(g, mtile, num_sms);
+    return launch_modal_pcg<double>(stream, modal, S, mtile, iters, d_err, kGridWaitLimit);
 }
 
 int Op::pcg_fp64(const double *b, const double *diag, double tol, int64_t max_iter, int check_every, double *x,
@@ -579,11 +608,18 @@ int Op::pcg_fp64(const double *b, const double *diag, double tol, int64_t max_it
         launches += 1;
     }
     inv_diag_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(ndof, diag, d_inv);
-    pcg_init_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(ndof, b, d_inv, d_x, d_r, d_p, d_partials);
+    pcg_init_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(ndof, b, d_inv, d_x, d_r, d_p, d_partials, nullptr, d_z);
     pcg_init_finalize<<<1, kVecThreads, 0, stream>>>(d_partials, vec_blocks, d_state, tol, max_iter);
     ICC_CUDA(cudaGetLastError(), "pcg init");
     if (check_every <= 0) check_every = 32;
-    if (!graph_exec || graph_batch != check_every) {
+    // the dense form replays a captured batch of iterations; the modal form iterates inside one launch and
+    // leaves it by itself, so the host looks less often
+    const int batch = modal.ok ? 8 * check_every : check_every;
+    if (modal.ok) {
+        ICC_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(unsigned long long), stream), "clear barrier");
+        ICC_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), stream), "clear err");
+        *h_err = 0;
+    } else if (!graph_exec || graph_batch != check_every) {
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
         graph_exec = nullptr;
         cudaGraph_t graph;
@@ -598,13 +634,16 @@ int Op::pcg_fp64(const double *b, const double *diag, double tol, int64_t max_it
     int64_t launched = 0;
     for (;;) {
         ICC_CUDA(cudaMemcpyAsync(h_state, d_state, sizeof(PcgState), cudaMemcpyDeviceToHost, stream), "state");
+        if (modal.ok) ICC_CUDA(cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "err");
         ICC_CUDA(cudaStreamSynchronize(stream), "pcg sync");
+        if (modal.ok && *h_err) return set_error(ICC_TIMEOUT, "pcg: grid barrier wait ran out");
         if (h_state->status != 0) break;
-        if (launched > max_iter + 2 * int64_t(check_every))
+        if (launched > max_iter + 2 * int64_t(batch))
             return set_error(ICC_TIMEOUT, "pcg: device state did not reach a stop condition");
-        ICC_CUDA(cudaGraphLaunch(graph_exec, stream), "graph launch");
-        launched += check_every;
-        launches += 4 * int64_t(check_every);
+        if (modal.ok) ICC_CUDA(enqueue_pcg_modal(batch), "pcg launch");
+        else ICC_CUDA(cudaGraphLaunch(graph_exec, stream), "graph launch");
+        launched += batch;
+        launches += modal.ok ? 1 : 4 * int64_t(check_every);
     }
     ICC_CUDA(cudaMemcpyAsync(x, d_x, (size_t)ndof * 8, cudaMemcpyDeviceToDevice, stream), "copy x");
     *iters = h_state->iter;

@@ -73,9 +73,8 @@ __device__ __forceinline__ void pcg_alpha_step(PcgState *st, double p_ap) {
     else st->alpha = st->rz_old / p_ap;
 }
 
-// relative residual test, then beta (rust/src/solver.rs:56-71)
-__device__ __forceinline__ void pcg_beta_step(PcgState *st, double rr, double rz) {
-    double res = sqrt(rr) / st->norm_b;
+// relative residual test, then beta (rust/src/solver.rs:56-71); res = |r| / |b|, beta = rz / rz_old
+__device__ __forceinline__ void pcg_beta_step(PcgState *st, double res, double rz, double beta) {
     st->rel_res = res;
     st->rz_prev = st->rz_old;  // the r'z of this iteration's alpha
     if (res < st->tol) {
@@ -83,11 +82,11 @@ __device__ __forceinline__ void pcg_beta_step(PcgState *st, double rr, double rz
     } else if (!isfinite(res)) {
         st->status = kStatNan;
     } else {
-        st->beta = rz / st->rz_old;
+        st->beta = beta;
         st->rz_old = rz;
         if (st->iter >= st->max_iter) st->status = kStatMaxIter;
-        else if (st->repl_delta > 0.0 && st->iter % st->repl_every == 0 &&
-                 (res < st->repl_delta * st->repl_res || st->iter - st->repl_iter >= st->repl_seg))
+        else if (st->repl_delta > 0.0 && (res < st->repl_delta * st->repl_res || st->iter - st->repl_iter >= st->repl_seg) &&
+                 st->iter % st->repl_every == 0)
             st->status = kStatReplace;
     }
 }
@@ -95,11 +94,11 @@ __device__ __forceinline__ void pcg_beta_step(PcgState *st, double rr, double rz
 // True in exactly one CTA: the last to finish.  Every CTA has stored its partial before calling;
 // the last one then reads all partials (in fixed order, so the result does not depend on which
 // CTA is last) and resets the counter for the next use.
-__device__ __forceinline__ bool last_block(unsigned *counter, unsigned total) {
+__device__ __forceinline__ bool last_block(unsigned *counter) {
     __shared__ bool is_last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) is_last = atomicAdd(counter, 1u) == total - 1u;
+    if (threadIdx.x == 0) is_last = atomicAdd(counter, 1u) == gridDim.x - 1;
     __syncthreads();
     if (is_last) {
         __threadfence();
@@ -117,6 +116,19 @@ __device__ __forceinline__ T sparse_row(const Sparse<T> &sp, long long idx, cons
     for (int k = sp.ptr[idx]; k < k1; ++k) {
         const int j = sp.idx[k];
         const T xj = (mask_mode != ICC_MASK_NONE && !mask[j]) ? T(0) : p[j];
+        acc += sp.val[k] * xj;
+    }
+    return acc;
+}
+
+// The same past the L1, for a direction that other CTAs of the running kernel wrote.
+template <class T>
+__device__ __forceinline__ T sparse_row_cg(const Sparse<T> &sp, long long idx, const T *p, const uint8_t *mask, int mask_mode) {
+    T acc = T(0);
+    const int k1 = sp.ptr[idx + 1];
+    for (int k = sp.ptr[idx]; k < k1; ++k) {
+        const int j = sp.idx[k];
+        const T xj = (mask_mode != ICC_MASK_NONE && !mask[j]) ? T(0) : __ldcg(p + j);
         acc += sp.val[k] * xj;
     }
     return acc;
@@ -159,7 +171,7 @@ gather_kernel(Geom g, Tiles t, const T *__restrict__ patch, const T *__restrict_
     if (partials) {
         dot = block_sum(dot);
         if (threadIdx.x == 0) partials[blockIdx.x] = dot;
-        if (fuse && last_block(counter, gridDim.x)) {
+        if (fuse && last_block(counter)) {
             double s2 = 0.0;
             for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x) s2 += __ldcg(partials + i);
             s2 = block_sum(s2);
@@ -177,18 +189,19 @@ __global__ void inv_diag_kernel(long long n, const double *__restrict__ d, T *__
 }
 
 // x = 0, r = b, z = D^-1 r, p = z; partials: r'z and b'b   (rust/src/solver.rs:15-36)
-// pmask != null keeps p zero on fixed DOFs (the mixed form's inner loop, ICC_MASK_ZERO)
+// pmask != null keeps p zero on fixed DOFs (the mixed form's inner loop, ICC_MASK_ZERO); z (modal form) may be null
 template <class T>
 __global__ void __launch_bounds__(kVecThreads)
 pcg_init_kernel(long long n, const T *__restrict__ b, const T *__restrict__ inv, T *__restrict__ x,
                 T *__restrict__ r, T *__restrict__ p, double *__restrict__ partials,
-                const uint8_t *__restrict__ pmask = nullptr) {
+                const uint8_t *__restrict__ pmask = nullptr, T *__restrict__ z = nullptr) {
     double rz = 0.0, bb = 0.0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         T bi = b[i], zi = inv[i] * bi;
         x[i] = T(0);
         r[i] = bi;
         p[i] = (pmask && !pmask[i]) ? T(0) : zi;
+        if (z) z[i] = zi;
         rz += double(bi) * double(zi);
         bb += double(bi) * double(bi);
     }
@@ -231,7 +244,7 @@ pcg_update_kernel(long long n, const T *__restrict__ p, const T *__restrict__ ap
         partials[2 * blockIdx.x] = rr;
         partials[2 * blockIdx.x + 1] = rz;
     }
-    if (fuse && last_block(counter, gridDim.x)) {
+    if (fuse && last_block(counter)) {
         double a = 0.0, c = 0.0;
         for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
             a += __ldcg(partials + 2 * i);
@@ -239,7 +252,7 @@ pcg_update_kernel(long long n, const T *__restrict__ p, const T *__restrict__ ap
         }
         a = block_sum(a);
         c = block_sum(c);
-        if (threadIdx.x == 0) pcg_beta_step(fuse, a, c);
+        if (threadIdx.x == 0) pcg_beta_step(fuse, sqrt(a) / fuse->norm_b, c, c / fuse->rz_old);
     }
 }
 
