@@ -273,7 +273,7 @@ class MatrixFreeOperator:
         return y
 
     def matvec_f32(self, x):
-        """FP32 tensor-core apply (the mixed form's inner operator)."""
+        """FP32 apply (the mixed form's inner operator)."""
         y = np.zeros(self.n, dtype=np.float32)
         _check(lib().icc_op_apply_f32(self._h, np.ascontiguousarray(x, dtype=np.float32), y, self.n))
         return y
@@ -298,7 +298,7 @@ class MatrixFreeOperator:
         return a.value, g.value
 
     def profile_apply_f32(self, x_ptr, y_ptr, reps=20):
-        """Mean device ms of (tensor-core brick kernel, node-sum kernel) over reps FP32 applies."""
+        """Mean device ms of (element kernel, node-sum kernel) over reps FP32 applies."""
         a, g = C.c_double(), C.c_double()
         _check(lib().icc_op_profile_apply_f32(self._h, C.c_void_p(x_ptr), C.c_void_p(y_ptr), reps, C.byref(a),
                                               C.byref(g)))
@@ -325,7 +325,7 @@ class PcgSolver:
     """rust/src/solver.rs:9-76 PcgSolver on the device operator.
 
     precision FP64 reproduces the reference loop in FP64; MIXED runs FP64 iterative refinement
-    around a tensor-core FP32 inner PCG.  ``solve`` returns (x, iters, rel_res) like the
+    around an FP32 inner PCG.  ``solve`` returns (x, iters, rel_res) like the
     reference; ``status`` holds the C status (ICC_OK, ICC_NOT_CONVERGED, ICC_BREAKDOWN).
     """
 
@@ -412,7 +412,8 @@ class CantileverTopOpt:
 
     def set_loads(self, forces):
         """Load cases (rows of forces, each of ndof).  In the mixed precision their state solves run as
-        one batch (one tensor-core apply over all cases per PCG iteration); in FP64 one after another."""
+        one batch (one tensor-core apply over all cases per PCG iteration); in FP64, and from 2^18
+        elements on, one after another."""
         f = np.ascontiguousarray(np.atleast_2d(forces), dtype=np.float64)
         _check(lib().icc_topopt_set_loads(self._h, f.shape[0], f.reshape(-1)))
 

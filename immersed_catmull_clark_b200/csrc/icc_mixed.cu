@@ -1,6 +1,12 @@
-// Mixed-precision form of the solve: a Jacobi-PCG whose iterations run in FP32 on the
-// 5th-generation tensor cores, with FP64 reductions, an FP64 solution and FP64 residual
-// replacement (reliable updates).
+// Mixed-precision form of the solve: a Jacobi-PCG whose iterations run in FP32, with FP64
+// reductions, an FP64 solution and FP64 residual replacement (reliable updates).
+//
+// Two forms of the iteration.  A solve of one system whose element matrices have the modal form runs in
+// icc_modal.cuh's persistent kernel, many iterations a launch.  Other matrices, and batches of several
+// systems, run on the tensor-core kernels of this file, two launches an iteration: at 128x64x64 97 us an
+// iteration against 70, but a batch of 12 designs of 16x8x8 to 50x25x25 elements took 63 ms here and 77 to 87 ms in
+// one persistent kernel with the CTAs shared out: a system there has too few CTAs for a march, whose
+// steps follow one another, and all wait for the slowest between launches.
 //
 // Tensor-core brick apply (persistent, one CTA per SM, bricks of 8x4x4 elements; element m of a
 // brick = row m of the MMA tile = TMEM lane m):
@@ -13,7 +19,7 @@
 // order, and the node-side pass resolves the brick overlaps, as in the FP64 apply: no atomics,
 // bitwise reproducible.
 //
-// Solve (mixed_solve): the FP32 recurrence x, r, p, Ap (FP64 dot products) runs in CUDA graphs;
+// Solve (mixed_solve): the FP32 recurrence x, r, p, Ap (FP64 dot products) runs on the device;
 // the FP64 solution accumulates its updates and the FP64 true residual b - A x (FP64 apply)
 // replaces the FP32 residual whenever it has fallen by a factor delta; the solve stops on the
 // FP64 true residual.
@@ -1803,9 +1809,9 @@ static std::vector<int> share_ctas(const std::vector<MixedItem> &items, int cap,
     return n;
 }
 
-// Runs the graph batches of a (batched) mixed solve until every system has stopped.
+// Runs the launches of a (batched) mixed solve until every system has stopped.
 //
-// Reliable-update PCG per system: the Jacobi-PCG recurrence runs in FP32 on the tensor-core
+// Reliable-update PCG per system: the Jacobi-PCG recurrence runs in FP32 on the FP32
 // operator; whenever its residual has fallen by `delta` since the last replacement (or below tol),
 // the FP32 solution increment is folded into the FP64 solution, the true residual b - A x is
 // recomputed with the FP64 operator, and the FP32 residual is replaced by it while the search
@@ -2195,6 +2201,12 @@ static int autotune(MixedBatch &bt, std::vector<MixedItem> &items, int max_per_s
     return rc;
 }
 
+// Elements from which the systems of a batch are solved one after another on the modal kernel instead of
+// together on the tensor-core kernels: such a system fills the chip by itself, and its iterations are shorter
+// (70 us against 97 at 128x64x64).  Measured, together and one after another: 4 systems of 80x40x40 143 and 161 ms, of
+// 96x48x48 210 and 204 ms, of 128x64x64 660 and 485 ms.
+constexpr long long kSoloElements = 1LL << 18;
+
 // Several systems at once: systems m of the call are (ops[m], vsets[m]) with right-hand side b[m]
 // (device), Jacobi diagonal diag[m] (device, null: the operator's own), tolerance tol[m] and
 // budget max_iter[m]; solutions into x[m] (device).  All operators must be on one device and have
@@ -2215,7 +2227,7 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
         ICC_CUDA(cudaStreamSynchronize(op->stream), "batch: drain handle");
     }
     // every system's K_u must be the first one's times a factor (elements of one shape)
-    bool modal = m == 1;
+    bool modal = true;
     for (Op *op : ops) modal = modal && op->modal.ok;
     if (!modal)
         for (size_t i = 0; i < m; ++i)
@@ -2252,7 +2264,6 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
         items[i].max_iter = max_iter[i];
         items[i].x_out = x[i];
         items[i].kfac = kfac[i];
-        if (!modal) append_descs(*ops[i], (int)i, descs);
         nbricks += ops[i]->g.nbricks;
     }
     if ((nbricks + ops[0]->num_sms - 1) / ops[0]->num_sms > kMaxListPerCta)
@@ -2260,6 +2271,50 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
     const int cap = tail_capacity(*ops[0]);
     if ((int)m > cap || (int)m > kMaxInst)
         return set_error(ICC_BAD_ARG, "batched mixed solve: more systems than resident CTAs of the vector step");
+    if (modal && m > 1) {
+        // systems that fill the chip go one after another on the modal kernel, the others together
+        std::vector<size_t> together;
+        auto part = [&](const std::vector<size_t> &idx) {
+            std::vector<Op *> o;
+            std::vector<VecSet *> v;
+            std::vector<const double *> bb, dd;
+            std::vector<double *> xx;
+            std::vector<double> tt, rr(idx.size());
+            std::vector<int64_t> mi, it(idx.size()), re(idx.size());
+            std::vector<int> st(idx.size());
+            for (size_t i : idx) {
+                o.push_back(ops[i]);
+                v.push_back(vsets[i]);
+                bb.push_back(b[i]);
+                dd.push_back(diag ? diag[i] : nullptr);
+                xx.push_back(x[i]);
+                tt.push_back(tol[i]);
+                mi.push_back(max_iter[i]);
+            }
+            const int prc = mixed_solve_batch(stream, o, v, bb.data(), dd.data(), tt.data(), mi.data(), opts, xx.data(), st.data(),
+                                              it.data(), rr.data(), re.data());
+            if (prc) return prc;
+            for (size_t k = 0; k < idx.size(); ++k) {
+                if (status) status[idx[k]] = st[k];
+                if (iters) iters[idx[k]] = it[k];
+                if (rel_res) rel_res[idx[k]] = rr[k];
+                if (replacements) replacements[idx[k]] = re[k];
+            }
+            return (int)ICC_OK;
+        };
+        for (size_t i = 0; i < m; ++i)
+            if (ops[i]->nel < kSoloElements) together.push_back(i);
+        if (together.size() < m) {
+            for (size_t i = 0; i < m; ++i)
+                if (ops[i]->nel >= kSoloElements && (rc = part({i}))) return rc;
+            return together.empty() ? ICC_OK : part(together);
+        }
+        modal = false;
+        for (size_t i = 0; i < m; ++i)
+            if ((rc = mixed_init_tc(*ops[i])) || (rc = vecset_tc(*ops[i], *vsets[i]))) return rc;
+    }
+    if (!modal)
+        for (size_t i = 0; i < m; ++i) append_descs(*ops[i], (int)i, descs);
     MixedBatch bt;
     bt.owned = true;
     bt.stream = stream;

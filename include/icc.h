@@ -41,8 +41,8 @@ extern "C" {
 
 /* ---- precision forms of the solve ---------------------------------------------------------- */
 #define ICC_FP64 0            /* all-FP64 apply, vectors and reductions */
-#define ICC_MIXED 1           /* Jacobi-PCG whose iterations run in FP32 on the tensor-core apply (a
-                                 3-term split-TF32 product) with FP64 reductions, an FP64 solution and
+#define ICC_MIXED 1           /* Jacobi-PCG whose iterations run in FP32 (the operator in Legendre modes,
+                                 or a 3-term split-TF32 tensor-core product) with FP64 reductions, an FP64 solution and
                                  FP64 residual replacement (reliable updates); stops on the FP64 true
                                  residual */
 
@@ -66,7 +66,7 @@ typedef struct icc_solve_info {
                                  rust/src/solver.rs:56-58; true FP64 residual for ICC_MIXED) */
     double device_ms;         /* device time of the solve (CUDA events on the handle's stream) */
     int64_t fp64_applies;     /* FP64 operator applications */
-    int64_t mixed_applies;    /* tensor-core (split-TF32) operator applications */
+    int64_t mixed_applies;    /* FP32 operator applications */
     int64_t kernel_launches;  /* kernels this library launched for the solve */
 } icc_solve_info;
 
@@ -82,7 +82,7 @@ void icc_space_destroy(icc_space *sp);
  * solve): elements [e0[d], e1[d]) per direction, 0 <= e0 < e1 <= nel_dir, with the parent's
  * B-splines, numbered locally (control points [e0, e1 + 2) of the parent, x fastest).  Its element
  * matrices (icc_element_matrices) are the parent's elements' matrices, including next to the cut,
- * and operators on it run on the tensor cores as well. */
+ * and operators on it take the same kernels. */
 int icc_space_window(const icc_space *sp, const int64_t e0[3], const int64_t e1[3], icc_space **out);
 /* ndof, nel, control points per direction, elements per direction */
 int icc_space_dims(const icc_space *sp, int64_t *ndof, int64_t *nel, int64_t ndof_dir[3], int64_t nel_dir[3]);
@@ -118,7 +118,7 @@ int icc_op_update_mask(icc_op *op, const uint8_t *free_mask, int32_t mask_mode);
  * assembled into the stiffness).  Triplets (row, col, value) over the DOF numbering, duplicates
  * summed (CsrMatrix::from_triplets, rust/src/sparse.rs:16-58); count = 0 removes the term.  The
  * diagonal (icc_op_diagonal, and the solve's default preconditioner) includes S's diagonal; the
- * FP64 forms apply S in FP64, the tensor-core FP32 form in FP32.  Element energies stay those of
+ * FP64 forms apply S in FP64, the FP32 form in FP32.  Element energies stay those of
  * K alone (as the reference computes them from the element matrices). */
 int icc_op_set_extra_triplets(icc_op *op, int64_t count, const int64_t *rows, const int64_t *cols,
                               const double *vals);
@@ -127,8 +127,9 @@ int icc_op_set_extra_triplets(icc_op *op, int64_t count, const int64_t *rows, co
 int icc_op_apply(icc_op *op, const double *x, double *y, int64_t n);
 /* Same on device arrays, enqueued on the handle's stream (see icc_op_stream). */
 int icc_op_apply_dev(icc_op *op, const double *x_dev, double *y_dev, int64_t n);
-/* y = A x in FP32 with the tensor-core contraction (3-term split-TF32 products, FP32
- * accumulation): the operator of the ICC_MIXED inner solve.  Host arrays / device arrays. */
+/* y = A x in FP32: in the element's Legendre modes where the element matrices have that form
+ * (isotropic elasticity), else 3-term split-TF32 tensor-core products: the operator of the
+ * ICC_MIXED inner solve.  Host arrays / device arrays. */
 int icc_op_apply_f32(icc_op *op, const float *x, float *y, int64_t n);
 int icc_op_apply_f32_dev(icc_op *op, const float *x_dev, float *y_dev, int64_t n);
 /* CsrMatrix::diagonal (rust/src/sparse.rs:70-78) of the unmasked operator: sum_e s_e K[a,a],
@@ -168,7 +169,8 @@ int icc_apply_f64_noalloc(const int64_t nel_dir[3], const double *ke_types_dev, 
 
 /* Many independent solves (designs of uneven sizes, or load cases) at once: instance i solves
  * ops[i] x[i] = b[i] as icc_pcg_solve does (diag may be NULL, or diag[i] NULL), all instances in
- * flight together on their handles' streams.  Per instance: status[i] (an icc_pcg_solve code),
+ * flight together on their handles' streams (ICC_MIXED: instances of 2^18 or more elements one
+ * after another, the others in one batch).  Per instance: status[i] (an icc_pcg_solve code),
  * iters[i], rel_res[i] (both may be NULL).  Returns ICC_OK when every instance ran (converged or
  * not), else the first instance's error.  The handles must be distinct. */
 int icc_pcg_solve_batched(int32_t count, icc_op *const *ops, const double *const *b, const double *const *diag,
@@ -206,9 +208,9 @@ void icc_topopt_destroy(icc_topopt *t);
 /* Several load cases (extends the reference's single tip load, which the handle starts with):
  * forces is nload x ndof (component-blocked, like every vector here).  Each design iteration then
  * solves every case warm-started from its previous state.  With cfg.precision = ICC_MIXED and
- * nload > 1 the cases' state solves run as one batch: every PCG iteration is one tensor-core
- * apply over the bricks of all cases and one fused vector step (per-case PCG scalars, each case
- * stops on its own tolerance).  With ICC_FP64 the cases are solved one after another.
+ * nload > 1 the cases' state solves run as one batch (from 2^18 elements on one after another):
+ * every PCG iteration is one tensor-core apply over the bricks of all cases and one fused vector
+ * step (per-case PCG scalars, each case stops on its own tolerance).  With ICC_FP64 the cases are solved one after another.
  * Compliance and element energies are summed over the cases, and pcg_iters reports the sum. */
 int icc_topopt_set_loads(icc_topopt *t, int32_t nload, const double *forces);
 
@@ -249,11 +251,11 @@ int icc_legacy_stabilization(const icc_space *sp, const int8_t *status, double g
 int icc_op_profile_apply(icc_op *op, const double *x_dev, double *y_dev, int32_t reps, double *contract_ms,
                          double *gather_ms);
 
-/* The same for the tensor-core FP32 apply (unmasked input x_dev, FP32 device arrays). */
+/* The same for the FP32 apply (unmasked input x_dev, FP32 device arrays). */
 int icc_op_profile_apply_f32(icc_op *op, const float *x_dev, float *y_dev, int32_t reps, double *contract_ms,
                              double *gather_ms);
 
-/* Polls of a grid-wide barrier in the mixed solve's fused vector step before it gives up and the
+/* Polls of a grid-wide barrier in the mixed solve's kernels before it gives up and the
  * solve returns ICC_TIMEOUT (default 2^22).  The error flag and the barrier counter are cleared at
  * the start of every call, so the handle works normally after a time-out.  Lets a test make the
  * bounded wait run out without a fault; no reference counterpart. */

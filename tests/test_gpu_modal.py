@@ -110,3 +110,25 @@ def test_modal_solve_residual(nel, mode, extra):
         assert np.linalg.norm(b - y) < 1.1 * tol * np.linalg.norm(b)
         x2, its2, _ = solver.solve(sp.ndof, b, None, op)
         assert its2 == its and np.array_equal(x2, x)   # bitwise reproducible
+
+
+def test_batch_of_large_and_small_systems():
+    """Systems of a batch on either side of the size from which they are solved one by one, two of them large:
+    the true residual of each by the oracle."""
+    tol = 1e-8
+    ops, bs, parts = [], [], []
+    for i, nel in enumerate([(24, 12, 12), (128, 64, 33), (13, 5, 7), (64, 64, 64)]):
+        bounds = ((0.0, float(nel[0])), (0.0, float(nel[1])), (0.0, float(nel[2])))
+        sp, osp = icc.SpaceBox(bounds, nel, 2), O.Space(bounds, nel, 2)
+        em = icc.elasticity_element_matrices(sp, *icc.lame(1.0 + i, 0.3))
+        rng = np.random.default_rng(i)
+        s = rng.uniform(0.1, 1.0, sp.nel)
+        fm = (np.arange(sp.ndof) % (nel[0] + 2) != 0).astype(np.uint8)
+        ops.append(icc.MatrixFreeOperator(sp, em, s, fm, icc.MASK_ZERO))
+        bs.append(rng.standard_normal(sp.ndof) * fm)
+        parts.append((osp, em, s, fm))
+    xs, its, res, st = icc.solve_batched(ops, bs, tol=tol, precision=icc.MIXED)
+    for x, b, (osp, em, s, fm), k in zip(xs, bs, parts, st):
+        assert k == 0
+        y = oracle_apply(osp, em.types, em.type_id, s, x, fm, icc.MASK_ZERO)
+        assert np.linalg.norm(b - y) < 1.1 * tol * np.linalg.norm(b)
