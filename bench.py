@@ -5,19 +5,19 @@ Workload (default): the SIMP cantilever on 128 x 64 x 64 elements (1,698,840 DOF
 [0,2]x[0,1]x[0,1], densities i.i.d. U[0.01,1] smoothed by a 3x3x3 box filter (seeded PCG64),
 E0 = 1, E_min = 1e-9, nu = 0.3, SIMP penalty 3, x = 0 clamped, unit downward traction on x = 2.
 One step = one Jacobi-PCG solve to relative residual 1e-8 from x = 0, in the mixed-precision form
-(tensor-core split-TF32 FP32 iterations with FP64 residual replacement) by default; the plain FP64
+(FP32 iterations with FP64 residual replacement) by default; the plain FP64
 solve of the same system is timed beside it (config.vs_fp64).  --mode fp64 times the plain solve only.
 
 value    = DOF * iterations / device seconds of the solve, inputs resident in HBM (CUDA events on
            the solver's stream, L2 flushed between steps), summed over ranks (replicas).
 e2e      = the same metric through the host-pointer C ABI call (icc_op_update_scale +
            icc_pcg_solve): H2D of the step's scale and load, D2H of the solution, inside the timing.
-roofline = the dominant kernel: for the mixed form the tensor-core brick apply, algorithmic
-           2*81*81 flops per element (the three split-TF32 products are credited once) over its
-           mean CUDA-event duration against this run's cuBLAS TF32 GEMM (the MMA work it executes,
-           three products padded to 96 x 96, is reported beside it as executed_flops); for
-           --mode fp64 the FP64 DMMA brick apply, 2*81*81 flops per element against this run's
-           cuBLAS DGEMM.  roofline.iteration: the whole PCG iteration against HBM bandwidth,
+roofline = the dominant kernel: the operator in the element's Legendre modes (FP32 for the mixed form,
+           FP64 for --mode fp64), its plain launch over its mean CUDA-event duration.  It executes
+           about 1,400 operations per element (the transforms between control values and modes
+           and 222 entries instead of 81 x 81), set against this run's cuBLAS GEMM of the same type on
+           the same units (SGEMM without TF32, DGEMM); the dense product's 2*81*81 flops per element
+           it stands for are reported beside it as algorithmic_flops.  roofline.iteration: the whole PCG iteration against HBM bandwidth,
            algorithmic bytes per iteration over ms_per_step / iterations.
 cpu_baseline / --impl reference = the oracle (C restatement of the reference's CPU path:
            element-loop operator with OpenMP, serial PCG vector loops) on the host cores, a
@@ -91,7 +91,7 @@ def parse():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--workload", default="cantilever128", choices=sorted(WORKLOADS))
     ap.add_argument("--mode", default="mixed", choices=["fp64", "mixed"],
-                    help="mixed: the tensor-core solve, timed beside the plain FP64 solve; fp64: the plain solve only")
+                    help="mixed: FP32 iterations with FP64 residual replacement, timed beside the plain FP64 solve; fp64: the plain solve only")
     ap.add_argument("--cpu-seconds", type=float, default=15.0, help="CPU baseline sample budget")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-ref-solution", action="store_true", help="skip the tight FP64 error reference")
@@ -167,12 +167,12 @@ class ClockSampler:
         return {"sm_mhz": float(np.median(sm)), "sm_max_mhz": mx, "reasons": sorted(reasons), "samples": len(sm)}
 
 
-def gemm_peak(torch, dev, dtype, tf32=False):
-    """Measured tensor-core peak of this GPU for one GEMM type: cuBLAS through torch.matmul, 8192^3,
-    best of 5 (TFLOP/s).  float64 -> DGEMM; float32 with tf32=True -> TF32 tensor cores."""
+def gemm_peak(torch, dev, dtype):
+    """Measured peak of this GPU for one GEMM type: cuBLAS through torch.matmul, 8192^3, best of 5
+    (TFLOP/s).  float64 -> DGEMM; float32 -> SGEMM (no TF32)."""
     n = 8192
     old = torch.backends.cuda.matmul.allow_tf32
-    torch.backends.cuda.matmul.allow_tf32 = tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
     a = torch.randn(n, n, dtype=dtype, device=dev)
     b = torch.randn(n, n, dtype=dtype, device=dev)
     for _ in range(2):
@@ -321,7 +321,7 @@ def run_batched(args, wl):
     ms_bat64, (_, _, _, st64) = timed(batched64, 1)
     out = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
            "ms_per_step": float(np.mean(ms)), "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-           "dtype": "tf32x3+f32+f64", "data": "synthetic",
+           "dtype": "f32+f64", "data": "synthetic",
            "config": {"workload": f"{wl['count']} cantilever designs 2k x k x k, k ~ U{{{wl['kmin']}..{wl['kmax']}}}",
                       "total_ndof": int(ndofs.sum()), "ks": [int(k) for k in ks], "tol": TOL, "seed": SEED,
                       "mode": "batched mixed", "iterations_total": int(np.sum(its)),
@@ -368,7 +368,7 @@ def run_topopt(args, wl):
     work = float(ndof * np.sum(hm.pcg_iterations))
     out = {"metric": METRIC, "value": work / tm, "unit": UNIT, "n_gpus": 1, "steps": args.steps, "warmup": 0,
            "ms_per_step": tm / args.steps * 1e3, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-           "dtype": "tf32x3+f32+f64", "data": "synthetic",
+           "dtype": "f32+f64", "data": "synthetic",
            "config": {"workload": f"SIMP cantilever {nel[0]}x{nel[1]}x{nel[2]}, 4 tip load cases, warm starts",
                       "ndof": ndof, "design_iterations": args.steps, "tol": TOL,
                       "mixed": {"s_per_design_iteration": tm / args.steps, "compliance": hm.compliance.tolist(),
@@ -507,31 +507,25 @@ def run_ours(args):
                "mixed_iterations": iters, "speedup_time_to_tol": t_fp64 / t_mixed}
 
     # roofline of the dominant kernel, timed on the solver's stream
-    flops_el = 2.0 * 81 * 81
-    nbricks = int(np.prod([-(-d // b) for d, b in zip(sp.nel_dir, (8, 4, 4))]))
-    executed = None
+    flops = 2.0 * 81 * 81 * sp.nel   # algorithmic: one 81 x 81 product per element
+    executed = 1400.0 * sp.nel       # in Legendre modes
     if precision == icc.MIXED:
         y32 = torch.empty(n, dtype=torch.float32, device=dev)
         p32 = torch.from_numpy(np.random.default_rng(1).standard_normal(n)).to(dev).to(torch.float32)
         contract_ms, gather_ms = op.profile_apply_f32(p32.data_ptr(), y32.data_ptr(), 20)
-        flops = flops_el * sp.nel   # algorithmic: one 81 x 81 product per element
-        # executed MMA work: three split products of 128 x 96 x 96 per brick of 8 x 4 x 4 elements
-        executed = 3 * 2.0 * 128 * 96 * 96 * nbricks
-        peak = gemm_peak(torch, dev, torch.float32, tf32=True)
-        kname, tkey = "apply_tc_kernel (tcgen05 kind::tf32, 3-term split)", "apply_tc_kernel"
-        peak_src = ("measured in this run: cuBLAS TF32 GEMM (torch.matmul float32 with TF32 tensor cores, 8192^3); "
-                    "MEASURED_PEAKS.json has no TF32 figure")
+        peak = gemm_peak(torch, dev, torch.float32)
+        kname, tkey = "modal_march_kernel<float>", "modal_march_kernel<float>"
+        peak_src = ("measured in this run: cuBLAS SGEMM (torch.matmul float32 without TF32, 8192^3); "
+                    "MEASURED_PEAKS.json has no FP32 figure")
     else:
         y_dev = torch.empty_like(x_dev)
         p_dev = torch.from_numpy(np.random.default_rng(1).standard_normal(n)).to(dev)
         contract_ms, gather_ms = op.profile_apply(p_dev.data_ptr(), y_dev.data_ptr(), 20)
-        flops = flops_el * sp.nel
-        executed = 2.0 * 88 * 84 * sp.nel   # DMMA tiles: 81 padded to 84 (trial) x 88 (test)
         peak = gemm_peak(torch, dev, torch.float64)
-        kname, tkey = "apply_f64_kernel (FP64 DMMA)", "apply_f64_kernel"
+        kname, tkey = "modal_march_kernel<double>", "modal_march_kernel<double>"
         peak_src = ("measured in this run: cuBLAS DGEMM (torch.matmul float64 8192^3); "
                     "MEASURED_PEAKS.json has no FP64 figure")
-    achieved = flops / (contract_ms * 1e-3) / 1e12
+    achieved = executed / (contract_ms * 1e-3) / 1e12
     traffic, traffic_src = None, None
     tpath = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     if os.path.exists(tpath):
@@ -604,13 +598,13 @@ def run_ours(args):
             cfg["vs_fp64"] = cmp
         out = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                "warmup": args.warmup, "ms_per_step": t_ms_all / args.steps, "higher_is_better": True,
-               "scaling": "weak", "vs_baseline": None, "dtype": "f64" if precision == icc.FP64 else "tf32x3+f32+f64",
+               "scaling": "weak", "vs_baseline": None, "dtype": "f64" if precision == icc.FP64 else "f32+f64",
                "data": "synthetic", "config": cfg,
-               "roofline": {"bound": "tensor", "kernel": kname, "achieved": achieved, "peak": peak,
+               "roofline": {"bound": "compute", "kernel": kname, "achieved": achieved, "peak": peak,
                             "unit": "TFLOP/s", "frac": achieved / peak, "frac_of": "measured", "traffic": traffic,
                             "traffic_source": traffic_src,
                             "algorithmic_flops_per_launch": flops, "executed_flops_per_launch": executed,
-                            "executed_tflops": executed / (contract_ms * 1e-3) / 1e12,
+                            "algorithmic_tflops": flops / (contract_ms * 1e-3) / 1e12,
                             "launch_ms": contract_ms, "node_sum_kernel_ms": gather_ms, "peak_source": peak_src,
                             "iteration": {"bound": "hbm", "algorithmic_bytes": iter_bytes, "ms": ms_per_iter,
                                           "achieved_gbs": iter_gbs, "peak_gbs": hbm, "frac": iter_gbs / hbm,

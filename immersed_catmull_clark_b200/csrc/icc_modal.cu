@@ -22,7 +22,9 @@ namespace {
 void rows_by(const double *Ax, const double *Ay, const double *Az, double *M) {
     const double *A[3] = {Ax, Ay, Az};
     const int st[3] = {1, 3, 9};
-    for (int d = 0; d < 3; ++d)
+    const double unit[9] = {1.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 1.0};
+    for (int d = 0; d < 3; ++d) {
+        if (std::equal(unit, unit + 9, A[d])) continue;
         for (int i = 0; i < 81; ++i) {
             if ((i % 27) / st[d] % 3 != 0) continue;
             double *r0 = M + i * 81, *r1 = r0 + st[d] * 81, *r2 = r1 + st[d] * 81;
@@ -34,6 +36,7 @@ void rows_by(const double *Ax, const double *Ay, const double *Az, double *M) {
                 r2[j] = a[6] * u + a[7] * v + a[8] * w;
             }
         }
+    }
 }
 
 // out = L K L' with L = Az (x) Ay (x) Ax per component (81 x 81, row-major)
