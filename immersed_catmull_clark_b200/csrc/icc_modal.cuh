@@ -12,7 +12,7 @@
 // mean of means is formed from differences of control values, so its rounding error scales with
 // the variation over the element, not with |u|; the mean of means is never needed (K maps it to 0).
 //
-// An element so costs about 700 operations instead of 81^2 = 6,561 multiply-adds.
+// An element so costs about 1,400 operations instead of 2 x 81^2 = 13,122.
 #pragma once
 
 #include <type_traits>
@@ -156,6 +156,13 @@ __device__ __forceinline__ void march_sync() {
 // point.  With PCG the input is formed on the fly, p = z + beta p_old, written to p_new where the
 // tile owns the control point, and this thread's part of p'Ap is returned.  No atomics: bitwise
 // reproducible.  sm: march_smem values; tm: the warp's tensor memory.
+//
+// A column per thread shares the z direction's transforms along the march and leaves x and y to two cheap
+// exchanges.  It is bound by the issue of few warps: 1.8 (FP64) and 2.8 (FP32) instructions per clock
+// and SM of 4, as tensor memory holds the state of 256 and 512 columns (in registers it spills).  Measured at
+// 128x64x64, whole FP64 apply: dense DMMA contraction 375 us, this 65 us; two or four threads per column 77
+// to 94 us.  FP32 at 256x128x128: tensor-core contraction 635 us, this 333 us.  DRAM traffic is the input and
+// the scale once (19.5 and 10.6 MB at 128x64x64).
 template <class T, int NT, bool PCG, bool WHOLE>
 __device__ __forceinline__ double modal_march(const ModalK<T> &K, const ModalSys<T> &S, int tile, T *sm, uint32_t tm, T beta,
                                               const T *p_old, T *p_new) {
@@ -459,8 +466,10 @@ __device__ __forceinline__ double modal_march(const ModalK<T> &K, const ModalSys
 // The same product on a small tile, all its elements at once: 256 threads, four per element (one a parity
 // class), go through the directions one after the other in shared memory, six barriers in all.  A
 // march's steps follow one another, about 2 us each however few columns there are; on grids that give
-// an SM only a few cubes this is an order of magnitude sooner, on large ones its small tiles (3.4
+// an SM only a few cubes this is sooner, on large ones its small tiles (3.4
 // partial sums per control point) and its traffic through shared memory cost more than the march.
+// Bound by the latency of its phases where it is used.  Measured at 24x16x12, whole FP64 apply: dense DMMA
+// contraction 13.0 us, this 6.4 us; a PCG iteration on cubes 12.6 us, on marches 22 us.
 constexpr int kCube = 4, kCubeP = kCube + 2, kCubeThreads = 256;
 constexpr int kCubeU = 3 * kCubeP * kCubeP * kCubeP;                    // control values [c][z][y][x]
 constexpr int kCubeX = 9 * kCubeP * kCubeP * kCube;                     // x modes [v][c][z][y][ex]; row sums [c][i][z][y][ex]
