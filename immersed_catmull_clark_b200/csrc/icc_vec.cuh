@@ -216,12 +216,6 @@ pcg_init_kernel(long long n, const T *__restrict__ b, const T *__restrict__ inv,
 __global__ void __launch_bounds__(kVecThreads)
 pcg_init_finalize(const double *__restrict__ partials, int np, PcgState *st, double tol, long long max_iter);
 
-// p'Ap -> alpha, or breakdown (rust/src/solver.rs:41-51)
-__global__ void __launch_bounds__(kVecThreads) pcg_alpha_kernel(const double *__restrict__ partials, int np, PcgState *st);
-
-// relative residual test, then beta (rust/src/solver.rs:56-71)
-__global__ void __launch_bounds__(kVecThreads) pcg_beta_kernel(const double *__restrict__ partials, int np, PcgState *st);
-
 // x += alpha p; r -= alpha Ap; partials: r'r and r'z with z = D^-1 r (rust/src/solver.rs:52-66)
 template <class T>
 __global__ void __launch_bounds__(kVecThreads)
