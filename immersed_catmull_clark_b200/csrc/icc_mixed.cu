@@ -2058,12 +2058,13 @@ int mixed_solve(Op &op, const double *b, const double *diag, double tol, int64_t
     bt.num_sms = op.num_sms;
     bt.bmat = ms.d_bmat;
     bt.limit = ms.grid_wait_limit;
+    bt.graph = ms.graph;
     if (op.modal.ok) {
         if ((rc = set_modal(bt, op, ms.v))) return rc;
     } else if (!ms.graph || ms.graph_batch != check_every || ms.graph_limit != ms.grid_wait_limit) {
         const TcInst I = make_inst(op, ms.v, ms.d_state, 0, bt.tail_grid, 1.f);
         ICC_CUDA(cudaMemcpyAsync(bt.d_inst, &I, sizeof(TcInst), cudaMemcpyHostToDevice, op.stream), "instance table");
-        bt.graph = ms.graph;
+        ms.graph = nullptr;   // capture_graph destroys the previous one
         if ((rc = capture_graph(bt, check_every))) return rc;
         ms.graph = bt.graph;
         ms.graph_batch = check_every;

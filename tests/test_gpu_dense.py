@@ -1,0 +1,94 @@
+"""Element matrices that the Legendre-mode kernels do not take: the dense DMMA and tensor-core kernels.
+
+The elements are of one triclinic material, so every element matrix is the uniform one seen through its
+element's B-spline basis (which the tensor-core form asks for), but shear and normal strains couple (which
+the mode form excludes).  All results are compared with the oracle's element loop."""
+import numpy as np
+import pytest
+
+import immersed_catmull_clark_b200 as icc
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def kron3(x, y, z):
+    return np.kron(z, np.kron(y, x))
+
+
+def triclinic_types(bounds, nel, sp):
+    """(types, type_id): K[(i, a), (j, b)] = sum_pq C_ipjq int dN_a/dx_p dN_b/dx_q of the uniform B-splines, then
+    R K R' per type, R the end elements' B-splines N_0 = 2 B_0, N_1 = B_1 - B_0 in terms of the uniform ones."""
+    a = np.random.default_rng(3).standard_normal((6, 6))
+    voigt = np.array([[0, 5, 4], [5, 1, 3], [4, 3, 2]])
+    c = (np.eye(6) + a @ a.T / 6.0)[voigt][:, :, voigt]           # C[i, p, j, q]
+    g, w = np.polynomial.legendre.leggauss(3)
+    t, w = 0.5 * (g + 1.0), 0.5 * w
+    b0 = np.array([0.5 * (1 - t) ** 2, 0.5 + t - t * t, 0.5 * t * t])
+    b1 = np.array([t - 1.0, 1.0 - 2.0 * t, t])
+    m = []                                                        # m[d][s][r] = int (d/dx)^s B_a (d/dx)^r B_b dx
+    for d in range(3):
+        h = (bounds[d][1] - bounds[d][0]) / nel[d]
+        v = [b0, b1 / h]
+        m.append([[h * np.einsum("aq,bq,q->ab", v[s], v[r], w) for r in range(2)] for s in range(2)])
+    ku = np.zeros((3, 27, 3, 27))
+    for p in range(3):
+        for q in range(3):
+            gpq = kron3(*(m[d][int(p == d)][int(q == d)] for d in range(3)))
+            ku += np.einsum("ij,ab->iajb", c[:, p, :, q], gpq)
+    ku = ku.reshape(81, 81)
+    em = icc.elasticity_element_matrices(sp, 1.0, 1.0)
+    tid = np.asarray(em.type_id)
+    types = np.zeros((len(em.types), 81, 81))
+    for k in range(len(types)):
+        e = int(np.flatnonzero(tid == k)[0])
+        pos = (e % nel[0], e // nel[0] % nel[1], e // (nel[0] * nel[1]))
+        r = []
+        for d in range(3):
+            x = 2.0 if pos[d] == 0 else 1.0
+            y = 2.0 if pos[d] == nel[d] - 1 else 1.0
+            r.append(np.array([[x, 0.0, 0.0], [1.0 - x, 1.0, 1.0 - y], [0.0, 0.0, y]]))
+        rr = np.kron(np.eye(3), kron3(*r))
+        types[k] = rr @ ku @ rr.T
+    return types, tid
+
+
+def system(nel, mode, seed=0):
+    bounds = ((0.0, 1.0 * nel[0]), (0.0, 0.9 * nel[1]), (0.0, 1.2 * nel[2]))
+    sp, osp = icc.SpaceBox(bounds, nel, 2), O.Space(bounds, nel, 2)
+    types, tid = triclinic_types(bounds, nel, sp)
+    rng = np.random.default_rng(seed)
+    s = rng.uniform(0.1, 1.0, sp.nel)
+    fm = np.ones(sp.ndof, dtype=np.uint8)
+    fm[np.arange(sp.ndof) % (nel[0] + 2) == 0] = 0                # clamped at the first control plane along x
+    op = icc.MatrixFreeOperator(sp, icc.ElementMatrices(types, tid), s, None if mode == icc.MASK_NONE else fm, mode)
+
+    def apply(x):
+        y = O.mf_apply(osp, types, tid.astype(np.int64), s, x if mode == icc.MASK_NONE else fm * x,
+                       np.ones(sp.ndof, dtype=np.uint8), icc.MASK_NONE)
+        if mode == icc.MASK_ZERO:
+            return fm * y
+        return np.where(fm > 0, y, x) if mode == icc.MASK_IDENTITY else y
+
+    return sp, op, fm, apply, rng
+
+
+@pytest.mark.parametrize("precision", [icc.FP64, icc.MIXED])
+@pytest.mark.parametrize("mode", [icc.MASK_ZERO, icc.MASK_IDENTITY])
+@pytest.mark.parametrize("nel", [(1, 1, 1), (9, 5, 6), (24, 12, 10)])
+def test_solve_twice_on_one_handle(nel, mode, precision):
+    """The second solve replays the iterations that the first one captured.  The FP64 recurrence's residual drifts by
+    about iterations x eps x |A||x|/|b| < 1e3 x 2e-16 x 1e4; the mixed solve stops on the true one."""
+    tol = 1e-8
+    sp, op, fm, apply, rng = system(nel, mode)
+    b = rng.standard_normal(sp.ndof) * fm
+    solver = icc.PcgSolver(5000, tol, precision=precision)
+    x, its, res = solver.solve(sp.ndof, b, None, op)
+    assert solver.status == icc.ICC_OK and res < tol
+    assert np.linalg.norm(b - apply(x)) < 1.1 * tol * np.linalg.norm(b)
+    assert op.last_solve_info().kernel_launches > 2 * its         # launches per iteration: not the mode kernel
+    x2, its2, _ = solver.solve(sp.ndof, b, None, op)
+    assert its2 == its and np.array_equal(x2, x)
+    b2 = rng.standard_normal(sp.ndof) * fm                        # another load on the captured iterations
+    x3, _, _ = solver.solve(sp.ndof, b2, None, op)
+    assert np.linalg.norm(b2 - apply(x3)) < 1.1 * tol * np.linalg.norm(b2)
