@@ -16,6 +16,7 @@ HEADERS = ["icc_internal.h", "icc_device.cuh", "icc_vec.cuh", "icc_modal.cuh", "
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
+    "-diag-error", "2809",            # a dropped launch status ([[nodiscard]]) fails the build
     "-Xcompiler", "-fPIC", "-shared",
     "-I", os.path.join(ROOT, "include"),
 ]

@@ -203,15 +203,16 @@ struct Op {
     int set_scale_dev(const double *scale_dev);   // device array, stream-ordered
     int set_mask(const uint8_t *free_mask, int mode);
     int set_extra(int64_t count, const int64_t *rows, const int64_t *cols, const double *vals);
-    cudaError_t enqueue_contract(cudaStream_t s, const double *x, const PcgState *st);
-    void enqueue_apply(const double *x, double *y, double *partials, const PcgState *st);
-    void enqueue_apply_on(cudaStream_t s, const double *x, double *y);   // y = A x on stream s
+    // a kernel that was not launched leaves old values behind, so no status of these may be dropped
+    [[nodiscard]] cudaError_t enqueue_contract(cudaStream_t s, const double *x, const PcgState *st);
+    [[nodiscard]] cudaError_t enqueue_apply(const double *x, double *y, double *partials, const PcgState *st);
+    [[nodiscard]] cudaError_t enqueue_apply_on(cudaStream_t s, const double *x, double *y);   // y = A x on stream s
     void enqueue_diagonal(double *d, cudaStream_t s);                     // the diagonal on stream s
     int apply_dev(const double *x, double *y);
     int diagonal_dev(double *d);
     int ensure_pcg_buffers();
-    void enqueue_pcg_iteration();
-    cudaError_t enqueue_pcg_modal(int iters);
+    [[nodiscard]] cudaError_t enqueue_pcg_iteration();
+    [[nodiscard]] cudaError_t enqueue_pcg_modal(int iters);
     int pcg_fp64(const double *b, const double *diag, double tol, int64_t max_iter, int check_every, double *x,
                  int64_t *iters, double *rel_res);
 };

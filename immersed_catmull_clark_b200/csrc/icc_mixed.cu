@@ -1939,7 +1939,7 @@ static int run_mixed(MixedBatch &bt, std::vector<MixedItem> &items, const icc_so
             Op &op = *it.op;
             VecSet &v = *it.v;
             ru_accumulate_kernel<<<op.vec_blocks, kVecThreads, 0, s>>>(op.ndof, v.x64, v.x32, it.nb);
-            op.enqueue_apply_on(s, v.x64, v.y64);
+            ICC_CUDA(op.enqueue_apply_on(s, v.x64, v.y64), "residual apply");
             ir_residual_kernel<<<op.vec_blocks, kVecThreads, 0, s>>>(op.ndof, it.b, v.y64, v.r64, op.d_partials);
             sum_partials_kernel<<<1, kVecThreads, 0, s>>>(op.d_partials, op.vec_blocks, bt.d_scalars, (int)i);
             launches += 5;

@@ -997,10 +997,10 @@ ModalK<T> modal_entries(const ModalHost &m);
 template <class T>
 ModalSys<T> modal_sys(const Op &op, const ModalTile &t);
 template <class T>
-cudaError_t launch_modal_apply(cudaStream_t s, const ModalHost &m, const ModalSys<T> &S, const ModalTile &t);
+[[nodiscard]] cudaError_t launch_modal_apply(cudaStream_t s, const ModalHost &m, const ModalSys<T> &S, const ModalTile &t);
 // `iters` iterations of a system on S.ncta CTAs, in the form of `t`.
 template <class T>
-cudaError_t launch_modal_pcg(cudaStream_t s, const ModalHost &m, const ModalSys<T> &S, const ModalTile &t, int iters, int *err,
-                             long long limit);
+[[nodiscard]] cudaError_t launch_modal_pcg(cudaStream_t s, const ModalHost &m, const ModalSys<T> &S, const ModalTile &t, int iters,
+                                           int *err, long long limit);
 
 }  // namespace icc

@@ -512,16 +512,20 @@ cudaError_t Op::enqueue_contract(cudaStream_t s, const double *x, const PcgState
 }
 
 // Enqueue y = A x on the op's stream (FP64).  partials != null also forms p'y per CTA.
-void Op::enqueue_apply(const double *x, double *y, double *partials, const PcgState *st) {
-    enqueue_contract(stream, x, st);
+cudaError_t Op::enqueue_apply(const double *x, double *y, double *partials, const PcgState *st) {
+    const cudaError_t e = enqueue_contract(stream, x, st);
+    if (e != cudaSuccess) return e;
     gather_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(g, tiles, d_patch, x, d_mask, mask_mode, extra64(), y,
                                                                   partials, st);
+    return cudaGetLastError();
 }
 
-void Op::enqueue_apply_on(cudaStream_t s, const double *x, double *y) {
-    enqueue_contract(s, x, nullptr);
+cudaError_t Op::enqueue_apply_on(cudaStream_t s, const double *x, double *y) {
+    const cudaError_t e = enqueue_contract(s, x, nullptr);
+    if (e != cudaSuccess) return e;
     gather_kernel<double><<<vec_blocks, kVecThreads, 0, s>>>(g, tiles, d_patch, x, d_mask, mask_mode, extra64(), y,
                                                              nullptr, nullptr);
+    return cudaGetLastError();
 }
 
 void Op::enqueue_diagonal(double *d, cudaStream_t s) {
@@ -529,8 +533,7 @@ void Op::enqueue_diagonal(double *d, cudaStream_t s) {
 }
 
 int Op::apply_dev(const double *x, double *y) {
-    enqueue_apply(x, y, nullptr, nullptr);
-    ICC_CUDA(cudaGetLastError(), "apply launch");
+    ICC_CUDA(enqueue_apply(x, y, nullptr, nullptr), "apply launch");
     return ICC_OK;
 }
 
@@ -566,13 +569,15 @@ int Op::ensure_pcg_buffers() {
 // on the first iteration, so p = z), Ap, alpha, x/r update, convergence test and the next beta.
 // Every kernel returns at once when the state says the solve has finished, so a batch may overrun
 // harmlessly.
-void Op::enqueue_pcg_iteration() {
+cudaError_t Op::enqueue_pcg_iteration() {
     pcg_p_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(ndof, d_r, d_inv, d_p, d_state);
-    enqueue_contract(stream, d_p, d_state);
+    const cudaError_t e = enqueue_contract(stream, d_p, d_state);   // reports a failed launch before it too
+    if (e != cudaSuccess) return e;
     gather_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(g, tiles, d_patch, d_p, d_mask, mask_mode, extra64(),
                                                                   d_ap, d_partials, d_state, d_state, d_counter);
     pcg_update_kernel<double><<<vec_blocks, kVecThreads, 0, stream>>>(ndof, d_p, d_ap, d_inv, d_x, d_r, d_partials,
                                                                       d_state, d_state, d_counter);
+    return cudaGetLastError();
 }
 
 // Iterations of the modal form in one launch, up to `iters` or until the solve stops.
@@ -624,8 +629,11 @@ int Op::pcg_fp64(const double *b, const double *diag, double tol, int64_t max_it
         graph_exec = nullptr;
         cudaGraph_t graph;
         ICC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-        for (int i = 0; i < check_every; ++i) enqueue_pcg_iteration();
-        ICC_CUDA(cudaStreamEndCapture(stream, &graph), "end capture");
+        cudaError_t ce = cudaSuccess;
+        for (int i = 0; i < check_every && ce == cudaSuccess; ++i) ce = enqueue_pcg_iteration();
+        const cudaError_t ee = cudaStreamEndCapture(stream, &graph);
+        ICC_CUDA(ce, "capture iteration");
+        ICC_CUDA(ee, "end capture");
         cudaError_t e = cudaGraphInstantiate(&graph_exec, graph, 0);
         cudaGraphDestroy(graph);
         ICC_CUDA(e, "graph instantiate");

@@ -281,7 +281,7 @@ static int solve_state_dev(icc_op *h, StateScratch &s, const double *force, cons
     const int nb = s.nblocks;
     const uint8_t *mask = o.mask_mode != ICC_MASK_NONE ? o.d_mask : nullptr;
     // K u0 on the free rows (the masked operator; u0 vanishes on fixed DOFs)
-    o.enqueue_apply(u0, s.ku0, nullptr, nullptr);
+    ICC_CUDA(o.enqueue_apply(u0, s.ku0, nullptr, nullptr), "state apply");
     state_rhs_kernel<<<nb, kTopoThreads, 0, o.stream>>>(n, force, s.ku0, mask, s.b, s.part);
     double nf2 = 0.0, rb2 = 0.0;
     if ((rc = reduce_to_host(o, s, s.part, nb, 0, &nf2))) return rc;
@@ -320,7 +320,7 @@ static int solve_states_batched(icc_op *h, StateScratch &s, int nload, const dou
     for (int k = 0; k < nload; ++k) {
         const double *fk = force + (size_t)k * n;
         double *uk = u + (size_t)k * n;
-        o.enqueue_apply(uk, s.ku0, nullptr, nullptr);
+        ICC_CUDA(o.enqueue_apply(uk, s.ku0, nullptr, nullptr), "state apply");
         state_rhs_kernel<<<nb, kTopoThreads, 0, o.stream>>>(n, fk, s.ku0, mask, bk + (size_t)k * n, s.part);
         double nf2 = 0.0, rb2 = 0.0;
         if ((rc = reduce_to_host(o, s, s.part, nb, 0, &nf2))) return rc;
