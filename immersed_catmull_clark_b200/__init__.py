@@ -312,7 +312,7 @@ class MatrixFreeOperator:
         return ee
 
     def set_wait_limit(self, grid_polls):
-        """Polls of a grid barrier in the mixed solve's fused vector step before ICC_TIMEOUT."""
+        """Polls of a grid barrier in a solve, of either precision, before ICC_TIMEOUT."""
         _check(lib().icc_op_set_wait_limit(self._h, int(grid_polls)))
 
     def last_solve_info(self):

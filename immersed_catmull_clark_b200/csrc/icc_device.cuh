@@ -139,6 +139,8 @@ struct ModalTile {
     Tiles t{};
 };
 
+constexpr long long kGridWaitLimit = 1LL << 22;   // default polls of a grid barrier before it gives up
+
 struct MixedState;  // tensor-core path (icc_mixed.cu)
 struct StateScratch;  // warm-started state solve and element energies (icc_topopt.cu)
 
@@ -182,6 +184,7 @@ struct Op {
     double *d_p2 = nullptr, *d_z = nullptr, *d_part_a = nullptr;
     unsigned long long *d_bar = nullptr;
     int *d_err = nullptr, *h_err = nullptr;
+    long long grid_wait_limit = kGridWaitLimit;   // of the solves in either precision
     PcgState *d_state = nullptr, *h_state = nullptr;
     unsigned *d_counter = nullptr;          // last-CTA counter of the fused reductions
     cudaGraphExec_t graph_exec = nullptr;
@@ -224,7 +227,6 @@ bool modal_setup(const Op &op, ModalHost &m);
 template <class T>
 ModalTile modal_tile(const Geom &g, int num_sms);
 int modal_ctas(const Geom &g, const ModalTile &t, int num_sms);
-constexpr long long kGridWaitLimit = 1LL << 22;   // default polls of a grid barrier before it gives up
 
 // tensor-core mixed-precision path (icc_mixed.cu)
 void mixed_release(Op &op);

@@ -132,7 +132,6 @@ struct MixedState {
     int *h_err = nullptr;                      // pinned copy of d_err read after every graph batch
     unsigned long long *d_grid_ctr = nullptr;  // grid barrier counter of the fused vector step
     int tail_per_sm = 1;                       // resident CTAs of the fused vector step per SM
-    long long grid_wait_limit = kGridWaitLimit;
     VecSet v;                                  // the handle's own system
     TcInst *d_inst = nullptr;                  // its one-entry instance table
     PcgState *d_state = nullptr, *h_state = nullptr;
@@ -1638,11 +1637,11 @@ void mixed_invalidate_graph(Op &op) {
     op.mixed->graph_batch = 0;
 }
 
-// Polls of a grid barrier before the fused vector step gives up (ICC_TIMEOUT).
+// Polls of a grid barrier before a solve gives up (ICC_TIMEOUT).
 int mixed_set_wait_limit(Op &op, long long polls) {
     int rc = mixed_init(op);
     if (rc) return rc;
-    op.mixed->grid_wait_limit = polls;
+    op.grid_wait_limit = polls;
     return ICC_OK;
 }
 
@@ -2057,18 +2056,18 @@ int mixed_solve(Op &op, const double *b, const double *diag, double tol, int64_t
     bt.tail_grid = share_ctas(items, tail_capacity(op))[0];
     bt.num_sms = op.num_sms;
     bt.bmat = ms.d_bmat;
-    bt.limit = ms.grid_wait_limit;
+    bt.limit = op.grid_wait_limit;
     bt.graph = ms.graph;
     if (op.modal.ok) {
         if ((rc = set_modal(bt, op, ms.v))) return rc;
-    } else if (!ms.graph || ms.graph_batch != check_every || ms.graph_limit != ms.grid_wait_limit) {
+    } else if (!ms.graph || ms.graph_batch != check_every || ms.graph_limit != op.grid_wait_limit) {
         const TcInst I = make_inst(op, ms.v, ms.d_state, 0, bt.tail_grid, 1.f);
         ICC_CUDA(cudaMemcpyAsync(bt.d_inst, &I, sizeof(TcInst), cudaMemcpyHostToDevice, op.stream), "instance table");
         ms.graph = nullptr;   // capture_graph destroys the previous one
         if ((rc = capture_graph(bt, check_every))) return rc;
         ms.graph = bt.graph;
         ms.graph_batch = check_every;
-        ms.graph_limit = ms.grid_wait_limit;
+        ms.graph_limit = op.grid_wait_limit;
     }
     int64_t launches = 0;
     rc = run_mixed(bt, items, opts, &launches);
@@ -2323,7 +2322,7 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
     bt.nbricks = nbricks;
     bt.num_sms = ops[0]->num_sms;
     bt.bmat = ops[0]->mixed->d_bmat;
-    bt.limit = ops[0]->mixed->grid_wait_limit;
+    bt.limit = ops[0]->grid_wait_limit;
     if ((rc = dalloc(&bt.d_inst, m, "alloc batch")) || (rc = dalloc(&bt.d_desc, descs.size(), "alloc batch")) ||
         (rc = dalloc(&bt.d_state, m, "alloc batch")) ||
         (rc = dalloc(&bt.d_scalars, m, "alloc batch")) || (rc = dalloc(&bt.d_err, 1, "alloc batch")) ||

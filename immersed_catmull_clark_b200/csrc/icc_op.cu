@@ -599,7 +599,7 @@ cudaError_t Op::enqueue_pcg_modal(int iters) {
     S.bar = d_bar;
     S.st = d_state;
     S.ncta = modal_ctas(g, mtile, num_sms);
-    return launch_modal_pcg<double>(stream, modal, S, mtile, iters, d_err, kGridWaitLimit);
+    return launch_modal_pcg<double>(stream, modal, S, mtile, iters, d_err, grid_wait_limit);
 }
 
 int Op::pcg_fp64(const double *b, const double *diag, double tol, int64_t max_iter, int check_every, double *x,
