@@ -1909,8 +1909,7 @@ static int run_mixed(MixedBatch &bt, std::vector<MixedItem> &items, const icc_so
 
     // the modal form leaves its launch by itself when it wants a replacement or stops
     const int batch = bt.modal ? 8 * check_every : check_every;
-    int64_t launched = 0, max_budget = 0;
-    for (const auto &it : items) max_budget = std::max(max_budget, it.max_iter);
+    std::vector<int64_t> seen(m, 0);   // iterations at the last look
     size_t active = 0;
     for (const auto &it : items) active += it.done ? 0 : 1;
     while (active > 0) {
@@ -1919,17 +1918,20 @@ static int run_mixed(MixedBatch &bt, std::vector<MixedItem> &items, const icc_so
                      "solve launch");
         else ICC_CUDA(cudaGraphLaunch(bt.graph, s), "graph launch");
         launches += bt.modal ? 1 : 2 * int64_t(check_every);
-        launched += batch;
         ICC_CUDA(cudaMemcpyAsync(bt.h_state, bt.d_state, m * sizeof(PcgState), cudaMemcpyDeviceToHost, s), "state");
         ICC_CUDA(cudaMemcpyAsync(bt.h_err, bt.d_err, sizeof(int), cudaMemcpyDeviceToHost, s), "err");
         ICC_CUDA(cudaStreamSynchronize(s), "inner sync");
         if (*bt.h_err) return timeout_error(*bt.h_err);   // a bounded wait ran out in this batch
         // systems that asked for a replacement or stopped: reliable update x += sigma xs, r = b - A x in FP64
         std::vector<size_t> upd;
-        for (size_t i = 0; i < m; ++i)
+        bool moved = false;
+        for (size_t i = 0; i < m; ++i) {
             if (!items[i].done && bt.h_state[i].status != 0) upd.push_back(i);
+            moved = moved || bt.h_state[i].iter > seen[i];
+            seen[i] = bt.h_state[i].iter;
+        }
         if (upd.empty()) {
-            if (launched > max_budget + 2 * int64_t(batch))
+            if (!moved)   // launches iterate until every active system stops or wants an update
                 return set_error(ICC_TIMEOUT, "mixed solve: device state did not reach a stop condition");
             continue;
         }

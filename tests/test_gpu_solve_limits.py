@@ -28,3 +28,13 @@ def test_fp64_grid_barrier_timeout_then_recovery():
     op.set_wait_limit(1 << 22)
     x2, its2, _ = solver.solve(sp.ndof, b, None, op)
     assert solver.status == icc.ICC_OK and its2 == its and np.array_equal(x2, x)
+
+
+@pytest.mark.parametrize("check", [1, 4, 16, 32])
+def test_iteration_budget_of_a_mixed_solve(check):
+    """A mixed solve that leaves its launches early, at residual replacements, still has its whole iteration budget:
+    it ends as not converged with every iteration spent, not as a time-out."""
+    p, sp, op = cantilever((53, 31, 27))
+    solver = icc.PcgSolver(1000, 1e-30, precision=icc.MIXED, check_every=check)
+    x, its, res = solver.solve(sp.ndof, W.rhs_masked(p), None, op)
+    assert solver.status == icc.ICC_NOT_CONVERGED and its == 1000
