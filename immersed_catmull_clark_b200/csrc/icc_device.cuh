@@ -227,6 +227,10 @@ bool modal_setup(const Op &op, ModalHost &m);
 template <class T>
 ModalTile modal_tile(const Geom &g, int num_sms);
 int modal_ctas(const Geom &g, const ModalTile &t, int num_sms);
+struct ModalRun {
+    int iters, launches;   // iterations of a launch, launches between two looks of the host
+};
+ModalRun modal_run(const Op &op, bool f64, int check_every);
 
 // tensor-core mixed-precision path (icc_mixed.cu)
 void mixed_release(Op &op);

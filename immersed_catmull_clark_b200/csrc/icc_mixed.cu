@@ -1907,17 +1907,17 @@ static int run_mixed(MixedBatch &bt, std::vector<MixedItem> &items, const icc_so
     int rc;
     if ((rc = init_items(bt, items, delta, check_every, false, launches))) return rc;
 
-    // the modal form leaves its launch by itself when it wants a replacement or stops
-    const int batch = bt.modal ? 8 * check_every : check_every;
+    const ModalRun run = bt.modal ? modal_run(*bt.modal, false, check_every) : ModalRun{};
     std::vector<int64_t> seen(m, 0);   // iterations at the last look
     size_t active = 0;
     for (const auto &it : items) active += it.done ? 0 : 1;
     while (active > 0) {
         if (bt.modal)
-            ICC_CUDA(launch_modal_pcg<float>(s, bt.modal->modal, bt.sys, bt.modal->mixed->mt, batch, bt.d_err, bt.limit),
-                     "solve launch");
+            for (int k = 0; k < run.launches; ++k)
+                ICC_CUDA(launch_modal_pcg<float>(s, bt.modal->modal, bt.sys, bt.modal->mixed->mt, run.iters, bt.d_err, bt.limit),
+                         "solve launch");
         else ICC_CUDA(cudaGraphLaunch(bt.graph, s), "graph launch");
-        launches += bt.modal ? 1 : 2 * int64_t(check_every);
+        launches += bt.modal ? run.launches : 2 * int64_t(check_every);
         ICC_CUDA(cudaMemcpyAsync(bt.h_state, bt.d_state, m * sizeof(PcgState), cudaMemcpyDeviceToHost, s), "state");
         ICC_CUDA(cudaMemcpyAsync(bt.h_err, bt.d_err, sizeof(int), cudaMemcpyDeviceToHost, s), "err");
         ICC_CUDA(cudaStreamSynchronize(s), "inner sync");

@@ -241,6 +241,21 @@ int modal_ctas(const Geom &g, const ModalTile &t, int num_sms) {
     return std::min(num_sms, std::max(t.t.n, (int)((g.nsc + 511) / 512)));
 }
 
+// A launch takes every SM, so work on other streams waits until it ends: about 8 ms of an FP64 solve and 16 of a
+// mixed one, by a model of an iteration's time (measured, us: FP64 12.6 at 24x16x12, 27 at 53x31x27, 105 at 128x64x64,
+// 161 at 96^3; FP32 12.4, 24, 70, 102; the sparse term by its bytes).  The cuts cost nothing that shows (152.9 ms FP64 and
+// 126.6 mixed at 128x64x64 with and without; mixed ones of 8 ms 0.15%).  The host looks after up to 16 launches of an
+// FP64 solve, which stops once and whose queued launches then return at once, and after each one of a mixed solve,
+// which leaves it for a replacement every 75 iterations or so.
+ModalRun modal_run(const Op &op, bool f64, int check_every) {
+    const double us = 12.5 + (f64 ? 1.8e-4 : 1.1e-4) * (double)op.nel + 5e-6 * (double)op.sp_nnz;
+    const double want = 8.0 * check_every;
+    ModalRun r;
+    r.iters = (int)std::fmax(1.0, std::fmin(std::fmin(want, 1e6), std::floor((f64 ? 8000.0 : 16000.0) / us)));
+    r.launches = (int)std::fmin(std::ceil(want / r.iters), f64 ? 16.0 : 1.0);
+    return r;
+}
+
 // ---- launches -------------------------------------------------------------------------------------
 
 template <class T>

@@ -983,6 +983,7 @@ modal_pcg_kernel(const __grid_constant__ ModalK<T> K, const __grid_constant__ Mo
     }
     if (bid == 0 && tid == 0) {
         st.bars = (long long)bars;
+        if (*(volatile int *)err) st.status = kStatNan;   // a wait ran out: ends the launches queued behind this one too
         *S.st = st;
     }
     __syncthreads();

@@ -619,7 +619,8 @@ int Op::pcg_fp64(const double *b, const double *diag, double tol, int64_t max_it
     if (check_every <= 0) check_every = 32;
     // the dense form replays a captured batch of iterations; the modal form iterates inside one launch and
     // leaves it by itself, so the host looks less often
-    const int batch = modal.ok ? 8 * check_every : check_every;
+    const ModalRun run = modal_run(*this, true, check_every);
+    const int64_t batch = modal.ok ? int64_t(run.iters) * run.launches : check_every;
     if (modal.ok) {
         ICC_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(unsigned long long), stream), "clear barrier");
         ICC_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), stream), "clear err");
@@ -646,12 +647,13 @@ int Op::pcg_fp64(const double *b, const double *diag, double tol, int64_t max_it
         ICC_CUDA(cudaStreamSynchronize(stream), "pcg sync");
         if (modal.ok && *h_err) return set_error(ICC_TIMEOUT, "pcg: grid barrier wait ran out");
         if (h_state->status != 0) break;
-        if (launched > max_iter + 2 * int64_t(batch))
+        if (launched > max_iter + 2 * batch)
             return set_error(ICC_TIMEOUT, "pcg: device state did not reach a stop condition");
-        if (modal.ok) ICC_CUDA(enqueue_pcg_modal(batch), "pcg launch");
+        if (modal.ok)
+            for (int k = 0; k < run.launches; ++k) ICC_CUDA(enqueue_pcg_modal(run.iters), "pcg launch");
         else ICC_CUDA(cudaGraphLaunch(graph_exec, stream), "graph launch");
         launched += batch;
-        launches += modal.ok ? 1 : 4 * int64_t(check_every);
+        launches += modal.ok ? run.launches : 4 * int64_t(check_every);
     }
     ICC_CUDA(cudaMemcpyAsync(x, d_x, (size_t)ndof * 8, cudaMemcpyDeviceToDevice, stream), "copy x");
     *iters = h_state->iter;

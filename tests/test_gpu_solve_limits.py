@@ -1,4 +1,4 @@
-"""Limits of a solve's launches: the bounded grid barrier."""
+"""Limits of a solve's launches: the bounded grid barrier, the iteration budget, the length of one launch."""
 import numpy as np
 import pytest
 
@@ -38,3 +38,30 @@ def test_iteration_budget_of_a_mixed_solve(check):
     solver = icc.PcgSolver(1000, 1e-30, precision=icc.MIXED, check_every=check)
     x, its, res = solver.solve(sp.ndof, W.rhs_masked(p), None, op)
     assert solver.status == icc.ICC_NOT_CONVERGED and its == 1000
+
+
+@pytest.mark.parametrize("precision,nel,check", [(icc.FP64, (128, 64, 64), 32), (icc.FP64, (96, 96, 96), 32),
+                                                 (icc.FP64, (128, 64, 64), 1000), (icc.MIXED, (96, 96, 96), 1000)])
+def test_a_launch_holds_the_chip_for_milliseconds(precision, nel, check):
+    """One launch takes every SM, so work on other streams waits for it: launches are cut at about 8 ms (FP64) or 16 ms
+    whatever the grid and the check interval.  Half as much again is allowed for the model of an iteration's time."""
+    p, sp, op = cantilever(nel)
+    solver = icc.PcgSolver(1000, 1e-30, precision=precision, check_every=check, inner_tol=1e-30)
+    solver.solve(sp.ndof, W.rhs_masked(p), None, op)
+    info = op.last_solve_info()
+    assert info.iterations == 1000
+    assert info.device_ms / info.kernel_launches < (12.0 if precision == icc.FP64 else 24.0)
+
+
+def test_launch_cuts_do_not_change_the_solve():
+    """The iterations are the same whatever the launches they run in."""
+    p, sp, op = cantilever((53, 31, 27))
+    b = W.rhs_masked(p)
+    for precision in (icc.FP64, icc.MIXED):
+        ref = None
+        for check in (16, 32, 1 << 30):   # the replacements of the mixed form fall on multiples of the interval
+            if precision == icc.MIXED and check != 32:
+                continue
+            x, its, res = icc.PcgSolver(3000, 1e-8, precision=precision, check_every=check).solve(sp.ndof, b, None, op)
+            ref = (x, its, res) if ref is None else ref
+            assert its == ref[1] and res == ref[2] and np.array_equal(x, ref[0])
