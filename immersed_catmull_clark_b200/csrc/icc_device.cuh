@@ -214,6 +214,7 @@ struct Op {
     int apply_dev(const double *x, double *y);
     int diagonal_dev(double *d);
     int ensure_pcg_buffers();
+    int ensure_fp64_buffers();
     [[nodiscard]] cudaError_t enqueue_pcg_iteration();
     [[nodiscard]] cudaError_t enqueue_pcg_modal(int iters);
     int pcg_fp64(const double *b, const double *diag, double tol, int64_t max_iter, int check_every, double *x,

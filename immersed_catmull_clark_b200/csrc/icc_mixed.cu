@@ -114,6 +114,7 @@ struct VecSet {
     // modal form: the other direction, z = D^-1 r and the tile partial sums
     float *p32b = nullptr, *z32 = nullptr, *mpatch = nullptr;
     size_t mpatch_cap = 0;
+    bool tc_ready = false;   // the tensor-core form's buffers and input map
 };
 
 struct MixedState {
@@ -1299,22 +1300,21 @@ static int vecset_alloc(const Op &op, VecSet &v, int part_cap) {
 
 // What only one of the two forms needs, allocated on its first use.
 static int vecset_tc(Op &op, VecSet &v) {
-    if (v.pin32) return ICC_OK;
+    if (v.tc_ready) return ICC_OK;
     int rc;
     if (!v.ap32 && (rc = dalloc(&v.ap32, (size_t)op.ndof, "alloc mixed"))) return rc;
-    if ((rc = dalloc(&v.patch32, (size_t)op.g.nbricks * 3 * kPVol, "alloc mixed"))) return rc;
+    if (!v.patch32 && (rc = dalloc(&v.patch32, (size_t)op.g.nbricks * 3 * kPVol, "alloc mixed"))) return rc;
     v.cxp = (op.g.cx + 3) & ~3;
     const size_t npad = (size_t)3 * v.cxp * op.g.cy * op.g.cz;
-    if ((rc = dalloc(&v.pin32, npad, "alloc mixed"))) return rc;
+    if (!v.pin32 && (rc = dalloc(&v.pin32, npad, "alloc mixed"))) return rc;
     ICC_CUDA(cudaMemsetAsync(v.pin32, 0, npad * sizeof(float), op.stream), "clear apply input");
     ICC_CUDA(cudaStreamSynchronize(op.stream), "clear apply input");
-    return encode_input_map(op, v);
+    if ((rc = encode_input_map(op, v))) return rc;
+    v.tc_ready = true;
+    return ICC_OK;
 }
-static int vecset_modal(Op &op, VecSet &v, const Tiles &t) {
+static int vecset_mpatch(VecSet &v, const Tiles &t) {   // all that a plain modal apply needs
     int rc;
-    if (!v.p32b && (rc = dalloc(&v.p32b, (size_t)op.ndof, "alloc mixed"))) return rc;
-    if (!v.z32 && (rc = dalloc(&v.z32, (size_t)op.ndof, "alloc mixed"))) return rc;
-    if (op.sp_nnz && !v.ap32 && (rc = dalloc(&v.ap32, (size_t)op.ndof, "alloc mixed"))) return rc;
     const size_t need = (size_t)t.n * t.vol;
     if (need > v.mpatch_cap) {
         if (v.mpatch) cudaFree(v.mpatch);
@@ -1324,6 +1324,13 @@ static int vecset_modal(Op &op, VecSet &v, const Tiles &t) {
         v.mpatch_cap = need;
     }
     return ICC_OK;
+}
+static int vecset_modal(Op &op, VecSet &v, const Tiles &t) {
+    int rc;
+    if (!v.p32b && (rc = dalloc(&v.p32b, (size_t)op.ndof, "alloc mixed"))) return rc;
+    if (!v.z32 && (rc = dalloc(&v.z32, (size_t)op.ndof, "alloc mixed"))) return rc;
+    if (op.sp_nnz && !v.ap32 && (rc = dalloc(&v.ap32, (size_t)op.ndof, "alloc mixed"))) return rc;
+    return vecset_mpatch(v, t);
 }
 
 static void vecset_free(VecSet &v) {
@@ -1429,7 +1436,7 @@ static int mixed_init(Op &op) {
     }
     if ((rc = dalloc(&ms.d_scale32, (size_t)op.nel, "alloc mixed"))) return rc;
     if ((rc = vecset_alloc(op, ms.v, tail_capacity(op)))) return rc;
-    if ((rc = op.modal.ok ? vecset_modal(op, ms.v, ms.mt.t) : vecset_tc(op, ms.v))) return rc;
+    if (!op.modal.ok && (rc = vecset_tc(op, ms.v))) return rc;
     if ((rc = dalloc(&ms.d_scalars, 8, "alloc mixed"))) return rc;
     if ((rc = dalloc(&ms.d_grid_ctr, 1, "alloc mixed"))) return rc;
     if ((rc = dalloc(&ms.d_err, 1, "alloc mixed"))) return rc;
@@ -1614,6 +1621,7 @@ int mixed_apply_f32(Op &op, const float *x, float *y) {
     if (rc) return rc;
     MixedState &ms = *op.mixed;
     if (op.modal.ok) {
+        if ((rc = vecset_mpatch(ms.v, ms.mt.t))) return rc;
         ICC_CUDA(enqueue_modal(op, x), "modal apply launch");
         gather_kernel<float><<<op.vec_blocks, kVecThreads, 0, op.stream>>>(op.g, ms.mt.t, ms.v.mpatch, x, op.d_mask,
                                                                            op.mask_mode, op.extra32(), y, nullptr, nullptr);
@@ -1652,6 +1660,7 @@ int mixed_profile_apply(Op &op, const float *x, float *y, int reps, double *cont
     MixedState &ms = *op.mixed;
     if ((rc = clear_flags(op.stream, ms.d_err, ms.d_grid_ctr))) return rc;
     const bool modal = op.modal.ok;
+    if (modal && (rc = vecset_mpatch(ms.v, ms.mt.t))) return rc;
     if (!modal) {
         enqueue_pad_input(op, ms.v, x, op.stream);
         const TcInst I = make_inst(op, ms.v, nullptr, 0, 0, 1.f);

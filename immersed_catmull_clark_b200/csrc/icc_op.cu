@@ -544,24 +544,31 @@ int Op::diagonal_dev(double *d) {
     return ICC_OK;
 }
 
+// Allocates what is not there yet (a call after one that ran out of memory goes on where that one stopped).
+template <class T>
+static int dev_need(T **p, size_t count) {
+    return *p ? ICC_OK : dev_alloc(p, count, "alloc pcg");
+}
+
+// Buffers of a solve in either precision.
 int Op::ensure_pcg_buffers() {
-    if (d_x) return ICC_OK;
+    double **v[] = {&d_x, &d_r, &d_p, &d_inv, &d_b, &d_diag};
     int rc;
-    if ((rc = dev_alloc(&d_x, (size_t)ndof, "alloc pcg"))) return rc;
-    if ((rc = dev_alloc(&d_r, (size_t)ndof, "alloc pcg"))) return rc;
-    if ((rc = dev_alloc(&d_p, (size_t)ndof, "alloc pcg"))) return rc;
-    if ((rc = dev_alloc(&d_ap, (size_t)ndof, "alloc pcg"))) return rc;
-    if (modal.ok) {
-        if ((rc = dev_alloc(&d_p2, (size_t)ndof, "alloc pcg"))) return rc;
-        if ((rc = dev_alloc(&d_z, (size_t)ndof, "alloc pcg"))) return rc;
-        if ((rc = dev_alloc(&d_part_a, (size_t)num_sms, "alloc pcg"))) return rc;
-        if ((rc = dev_alloc(&d_bar, 1, "alloc pcg"))) return rc;
-        if ((rc = dev_alloc(&d_err, 1, "alloc pcg"))) return rc;
-        ICC_CUDA(cudaMallocHost((void **)&h_err, sizeof(int)), "alloc pinned");
-    }
-    if ((rc = dev_alloc(&d_inv, (size_t)ndof, "alloc pcg"))) return rc;
-    if ((rc = dev_alloc(&d_b, (size_t)ndof, "alloc pcg"))) return rc;
-    if ((rc = dev_alloc(&d_diag, (size_t)ndof, "alloc pcg"))) return rc;
+    for (double **p : v)
+        if ((rc = dev_need(p, (size_t)ndof))) return rc;
+    return ICC_OK;
+}
+
+// Those of the FP64 solve alone.  The modal form stores Ap for a sparse term only.
+int Op::ensure_fp64_buffers() {
+    int rc;
+    if ((rc = ensure_pcg_buffers())) return rc;
+    if ((!modal.ok || sp_nnz) && (rc = dev_need(&d_ap, (size_t)ndof))) return rc;
+    if (!modal.ok) return ICC_OK;
+    if ((rc = dev_need(&d_p2, (size_t)ndof)) || (rc = dev_need(&d_z, (size_t)ndof)) ||
+        (rc = dev_need(&d_part_a, (size_t)num_sms)) || (rc = dev_need(&d_bar, 1)) || (rc = dev_need(&d_err, 1)))
+        return rc;
+    if (!h_err) ICC_CUDA(cudaMallocHost((void **)&h_err, sizeof(int)), "alloc pinned");
     return ICC_OK;
 }
 
@@ -605,7 +612,7 @@ cudaError_t Op::enqueue_pcg_modal(int iters) {
 int Op::pcg_fp64(const double *b, const double *diag, double tol, int64_t max_iter, int check_every, double *x,
                  int64_t *iters, double *rel_res) {
     int rc;
-    if ((rc = ensure_pcg_buffers())) return rc;
+    if ((rc = ensure_fp64_buffers())) return rc;
     int64_t launches = 3;
     if (!diag) {
         if ((rc = diagonal_dev(d_diag))) return rc;

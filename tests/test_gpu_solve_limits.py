@@ -1,6 +1,8 @@
-"""Limits of a solve's launches: the bounded grid barrier, the iteration budget, the length of one launch."""
+"""Limits of a solve's launches: the bounded grid barrier, the iteration budget, the length of one launch, device
+memory."""
 import numpy as np
 import pytest
+import torch
 
 import immersed_catmull_clark_b200 as icc
 from immersed_catmull_clark_b200 import workloads as W
@@ -65,3 +67,21 @@ def test_launch_cuts_do_not_change_the_solve():
             x, its, res = icc.PcgSolver(3000, 1e-8, precision=precision, check_every=check).solve(sp.ndof, b, None, op)
             ref = (x, its, res) if ref is None else ref
             assert its == ref[1] and res == ref[2] and np.array_equal(x, ref[0])
+
+
+def test_batch_memory():
+    """Systems of a batch that run on the tensor-core kernels hold no vectors of the other form."""
+    nel = (76, 56, 56)     # below the size from which a system is solved on its own
+    for k in range(2):     # the first batch also loads the kernels
+        inst = [cantilever(nel, seed=2 * k + i) for i in range(2)]
+        sp, ops, bs = inst[0][1], [i[2] for i in inst], [W.rhs_masked(i[0]) for i in inst]
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        icc.solve_batched(ops, bs, tol=1e-3, max_iter=64, precision=icc.MIXED)
+        used = free - torch.cuda.mem_get_info()[0]
+    n, bricks = sp.ndof, -(-nel[0] // 8) * -(-nel[1] // 4) * -(-nel[2] // 4)
+    padded = 3 * ((nel[0] + 2 + 3) // 4 * 4) * (nel[1] + 2) * (nel[2] + 2)
+    # FP64: x, r, p, Ap, D^-1, b, diagonal; x, r, y of the mixed form; FP32: load, x, r, p, Ap, D^-1, padded input, brick
+    # partial sums, scale.  Allocations are rounded up to 2 MB; the small ones of a handle share two such blocks.
+    sizes = [8 * n] * 10 + [4 * n] * 6 + [4 * padded, 4 * bricks * 3 * 360, 4 * sp.nel]
+    assert used <= 2 * sum(-(-s // (2 << 20)) for s in sizes) * (2 << 20) + 2 * (4 << 20)
