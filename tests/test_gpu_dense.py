@@ -92,3 +92,77 @@ def test_solve_twice_on_one_handle(nel, mode, precision):
     b2 = rng.standard_normal(sp.ndof) * fm                        # another load on the captured iterations
     x3, _, _ = solver.solve(sp.ndof, b2, None, op)
     assert np.linalg.norm(b2 - apply(x3)) < 1.1 * tol * np.linalg.norm(b2)
+
+
+def extra_term(sp, rng):
+    """Triplets of a symmetric, diagonally dominant sparse term."""
+    i = rng.permutation(sp.ndof)[: sp.ndof // 8 * 2].reshape(2, -1)
+    k = i.shape[1]
+    return (np.concatenate([i[0], i[1], i[0], i[1]]), np.concatenate([i[1], i[0], i[0], i[1]]),
+            np.concatenate([np.full(2 * k, -0.05), np.full(2 * k, 0.06)]))
+
+
+@pytest.mark.parametrize("extra", [False, True])
+@pytest.mark.parametrize("mode", [icc.MASK_NONE, icc.MASK_ZERO, icc.MASK_IDENTITY])
+@pytest.mark.parametrize("nel", [(1, 1, 1), (8, 4, 4), (9, 5, 6), (33, 17, 9)])
+def test_applies(nel, mode, extra):
+    """Both precisions, at sizes around the bricks of 8x4x4 elements; the repository's parity bars."""
+    sp, op, fm, apply, rng = system(nel, mode, seed=1)
+    r = c = np.zeros(0, dtype=np.int64)
+    v = np.zeros(0)
+    if extra:
+        r, c, v = extra_term(sp, rng)
+        op.set_extra_triplets(r, c, v)
+    w = v if mode == icc.MASK_NONE else v * fm[r] * fm[c]
+    x = rng.standard_normal(sp.ndof)
+    for a, y, tol in ((x, op.matvec(x), 1e-12), (x.astype(np.float32), op.matvec_f32(x.astype(np.float32)), 5e-6)):
+        ref = apply(a.astype(np.float64))
+        np.add.at(ref, r, w * a.astype(np.float64)[c])
+        assert np.linalg.norm(y - ref) < tol * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("precision", [icc.FP64, icc.MIXED])
+def test_solve_with_a_sparse_term(precision):
+    tol = 1e-8
+    sp, op, fm, apply, rng = system((17, 9, 10), icc.MASK_ZERO, seed=2)
+    b = rng.standard_normal(sp.ndof) * fm
+    solver = icc.PcgSolver(5000, tol, precision=precision)
+    solver.solve(sp.ndof, b, None, op)            # the captured iterations are rebuilt when the term is set
+    r, c, v = extra_term(sp, rng)
+    op.set_extra_triplets(r, c, v)
+    x, _, _ = solver.solve(sp.ndof, b, None, op)
+    y = apply(x)
+    np.add.at(y, r, v * fm[r] * fm[c] * x[c])
+    assert solver.status == icc.ICC_OK and np.linalg.norm(b - y) < 1.1 * tol * np.linalg.norm(b)
+
+
+def test_vector_step_timeout_then_recovery():
+    """The grid barrier of the tensor-core form's vector step runs out of polls; the handle solves normally
+    afterwards (its iterations were captured with the other limit)."""
+    sp, op, fm, apply, rng = system((16, 8, 8), icc.MASK_ZERO, seed=4)
+    b = rng.standard_normal(sp.ndof) * fm
+    solver = icc.PcgSolver(5000, 1e-8, precision=icc.MIXED)
+    op.set_wait_limit(0)   # no poll at all: every CTA that is not the last to arrive gives up
+    with pytest.raises(icc.IccError) as ei:
+        solver.solve(sp.ndof, b, None, op)
+    assert ei.value.code == icc.ICC_TIMEOUT
+    op.set_wait_limit(1 << 22)
+    x, _, _ = solver.solve(sp.ndof, b, None, op)
+    assert solver.status == icc.ICC_OK and np.linalg.norm(b - apply(x)) < 1.1e-8 * np.linalg.norm(b)
+
+
+def test_batch_of_both_kinds_of_matrices():
+    """Systems of the mode form in a batch with others: their elements differ in shape, which a batch refuses; each
+    kind alone is solved."""
+    sp, op, fm, apply, rng = system((9, 5, 6), icc.MASK_ZERO, seed=5)
+    iso = icc.MatrixFreeOperator(sp, icc.elasticity_element_matrices(sp, 1.0, 1.0), None, fm, icc.MASK_ZERO)
+    b = rng.standard_normal(sp.ndof) * fm
+    with pytest.raises(icc.IccError) as ei:
+        icc.solve_batched([op, iso], [b, b], tol=1e-8, precision=icc.MIXED)
+    assert ei.value.code == icc.ICC_BAD_ARG
+    sp2, op2, fm2, apply2, _ = system((24, 12, 10), icc.MASK_ZERO, seed=6)
+    b2 = rng.standard_normal(sp2.ndof) * fm2
+    xs, _, _, st = icc.solve_batched([op, op2], [b, b2], tol=1e-8, precision=icc.MIXED)
+    assert np.all(st == icc.ICC_OK)
+    for x, r, f in ((xs[0], b, apply), (xs[1], b2, apply2)):
+        assert np.linalg.norm(r - f(x)) < 1.1e-8 * np.linalg.norm(r)
