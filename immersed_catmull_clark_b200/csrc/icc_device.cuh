@@ -121,12 +121,6 @@ struct Edge {
     float e[3][4][4];   // e[d][a][b] = E[id a][id b]
 };
 
-__device__ __forceinline__ int edge_slot(const Edge &E, int d, int i) {
-    for (int a = 0; a < E.nb[d]; ++a)
-        if (E.id[d][a] == i) return a;
-    return -1;
-}
-
 // Element matrices in Legendre modes (icc_modal.cuh), when a handle's matrices have that form: the
 // entries, the end factors per direction and the uniform element matrix (81 x 81) they stand for.
 struct ModalHost {

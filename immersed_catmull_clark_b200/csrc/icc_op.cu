@@ -308,7 +308,7 @@ int Op::init(const Space &s, const double *ke_types, int nt, const int32_t *type
 
     if ((rc = dev_alloc(&d_scale, (size_t)nel, "alloc scale"))) return rc;
     if ((rc = dev_alloc(&d_mask, (size_t)ndof, "alloc mask"))) return rc;
-    if ((rc = dev_alloc(&d_patch, std::max((size_t)tiles.n * tiles.vol, (size_t)mtile.t.n * mtile.t.vol), "alloc patch scratch"))) return rc;
+    if ((rc = dev_alloc(&d_patch, (size_t)tiles.n * tiles.vol, "alloc patch scratch"))) return rc;
     if ((rc = dev_alloc(&d_x_in, (size_t)ndof, "alloc io"))) return rc;
     if ((rc = dev_alloc(&d_y_out, (size_t)ndof, "alloc io"))) return rc;
     vec_blocks = num_sms * 4;

@@ -104,93 +104,24 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
 }
 
 // N consecutive 32-bit TMEM columns of this thread's lane -> registers (asynchronous until tm_arrive) and
-// registers -> TMEM (until tmem_wait_st); warp w reaches lanes 32 (w % 4) .. + 31.
+// registers -> TMEM (until tmem_wait_st); warp w reaches lanes 32 (w % 4) .. + 31.  In pieces of two: a wider piece
+// wants its registers side by side.  The modal march in pieces of 2, 4 and 8, us: FP64 73.9, 76.2 and 74.2 at
+// 128x64x64, 51.7, 53.7 and 52.9 at 97x53x41; FP32 47.7, 47.4 and 47.4 at 128x64x64, 272, 266 and 265 at 256x128x128.
 template <int N>
-__device__ __forceinline__ void tm_ld(uint32_t taddr, uint32_t *r);
-template <int N>
-__device__ __forceinline__ void tm_st(uint32_t taddr, const uint32_t *r);
-template <>
-__device__ __forceinline__ void tm_ld<1>(uint32_t taddr, uint32_t *r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r[0]) : "r"(taddr) : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_st<1>(uint32_t taddr, const uint32_t *r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(r[0]) : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_ld<2>(uint32_t taddr, uint32_t *r) {
+__device__ __forceinline__ void tm_load(uint32_t taddr, uint32_t *r) {
+    static_assert(N % 2 == 0, "an even number of columns");
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];"
                  : "=r"(r[0]), "=r"(r[1])
                  : "r"(taddr) : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_st<2>(uint32_t taddr, const uint32_t *r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(taddr),
-                 "r"(r[0]), "r"(r[1])
-                 : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_ld<4>(uint32_t taddr, uint32_t *r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(taddr) : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_st<4>(uint32_t taddr, const uint32_t *r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr),
-                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
-                 : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_ld<8>(uint32_t taddr, uint32_t *r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr) : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_st<8>(uint32_t taddr, const uint32_t *r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
-                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_ld<16>(uint32_t taddr, uint32_t *r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_st<16>(uint32_t taddr, const uint32_t *r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-                 : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_ld<32>(uint32_t taddr, uint32_t *r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr) : "memory");
-}
-template <>
-__device__ __forceinline__ void tm_st<32>(uint32_t taddr, const uint32_t *r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
-                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-                 : "memory");
-}
-// any N in pieces of two: a wider piece wants its registers side by side, and the moves that puts them
-// there cost more than the instructions it saves (FP64 modal apply at 128x64x64: 425 moves a step)
-constexpr int kTmPiece = 2;
-template <int N>
-__device__ __forceinline__ void tm_load(uint32_t taddr, uint32_t *r) {
-    constexpr int P = kTmPiece < N ? kTmPiece : N;
-    tm_ld<P>(taddr, r);
-    if constexpr (N > P) tm_load<N - P>(taddr + P, r + P);
+    if constexpr (N > 2) tm_load<N - 2>(taddr + 2, r + 2);
 }
 template <int N>
 __device__ __forceinline__ void tm_store(uint32_t taddr, const uint32_t *r) {
-    constexpr int P = kTmPiece < N ? kTmPiece : N;
-    tm_st<P>(taddr, r);
-    if constexpr (N > P) tm_store<N - P>(taddr + P, r + P);
+    static_assert(N % 2 == 0, "an even number of columns");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(taddr),
+                 "r"(r[0]), "r"(r[1])
+                 : "memory");
+    if constexpr (N > 2) tm_store<N - 2>(taddr + 2, r + 2);
 }
 // waits for this thread's loads; the registers are tied to the wait, so no use moves before it
 template <int N>
@@ -200,16 +131,6 @@ __device__ __forceinline__ void tm_arrive(uint32_t *r) {
     for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
 }
 
-// 16 consecutive 32-bit TMEM columns of this thread's lane (warp w reads lanes 32w..32w+31).
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // 32 consecutive 32-bit TMEM columns of this thread's lane (asynchronous until tmem_wait_ld)
@@ -310,29 +231,16 @@ __device__ __forceinline__ bool named_sync_or(int id, int count, bool pred) {
     return r != 0;
 }
 
-// round to TF32 (10 explicit mantissa bits), nearest, ties away from zero
-__device__ __forceinline__ float to_tf32(float v) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
-    return __uint_as_float(r);
-}
-
-// The same rounding with two integer operations: add half of the dropped 13-bit field to the
-// magnitude and clear the field (finite inputs; a carry into the exponent is the correct result).
+// round to TF32 (10 explicit mantissa bits), nearest, ties away from zero, with two integer operations: add half
+// of the dropped 13-bit field to the magnitude and clear the field (finite inputs; a carry into the exponent is
+// the correct result)
 __device__ __forceinline__ float to_tf32_int(float v) {
     return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);
 }
 
-// v = hi + lo exactly up to the 13 bits dropped from lo: hi = tf32(v), lo = tf32(v - hi), where
-// v - hi is exact because hi is v rounded to 11 significant bits.
-__device__ __forceinline__ void split_tf32(float v, float &hi, float &lo) {
-    hi = to_tf32_int(v);
-    lo = to_tf32_int(v - hi);
-}
-
-// The same split with lo left in FP32 (v - hi is exact): a kind::tf32 MMA uses only the sign,
-// exponent and 10 leading mantissa bits of an operand, so lo enters the product with at most
-// 2^-10 |lo| <= 2^-21 |v| dropped, and the split costs three instructions instead of five.
+// v = hi + lo with hi = tf32(v) and lo = v - hi, which is exact because hi is v rounded to 11 significant bits.  lo
+// stays in FP32: a kind::tf32 MMA uses only the sign, exponent and 10 leading mantissa bits of an operand, so it
+// enters the product with at most 2^-10 |lo| <= 2^-21 |v| dropped, and the split costs three instructions.
 __device__ __forceinline__ void split_tf32_raw(float v, float &hi, float &lo) {
     hi = to_tf32_int(v);
     lo = v - hi;
