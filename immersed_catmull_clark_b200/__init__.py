@@ -413,7 +413,7 @@ class CantileverTopOpt:
     def set_loads(self, forces):
         """Load cases (rows of forces, each of ndof).  In the mixed precision their state solves run as
         one batch (one tensor-core apply over all cases per PCG iteration); in FP64, and from 2^18
-        elements on, one after another."""
+        elements on where that is sooner, one after another."""
         f = np.ascontiguousarray(np.atleast_2d(forces), dtype=np.float64)
         _check(lib().icc_topopt_set_loads(self._h, f.shape[0], f.reshape(-1)))
 

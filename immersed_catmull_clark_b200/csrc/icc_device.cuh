@@ -131,6 +131,7 @@ struct ModalHost {
 struct ModalTile {
     int nt = 0;   // columns of a march; 0: cubes of 4 x 4 x 4 elements
     Tiles t{};
+    double clocks = 0.0;   // of an apply, by the plan's model
 };
 
 constexpr long long kGridWaitLimit = 1LL << 22;   // default polls of a grid barrier before it gives up

@@ -2,9 +2,9 @@
 // reductions, an FP64 solution and FP64 residual replacement (reliable updates).
 //
 // Two forms of the iteration.  A solve of one system whose element matrices have the modal form runs in
-// icc_modal.cuh's persistent kernel, many iterations a launch.  Other matrices, and batches of several
-// systems, run on the tensor-core kernels of this file, two launches an iteration: at 128x64x64 97 us an
-// iteration against 70, but a batch of 12 designs of 16x8x8 to 50x25x25 elements took 63 ms here and 77 to 87 ms in
+// icc_modal.cuh's persistent kernel, many iterations a launch, unless its tiles fill the grid badly
+// (modal_sooner).  Other matrices, and batches of several systems, run on the tensor-core kernels of this file, two
+// launches an iteration: at 128x64x64 97 us an iteration against 70, but a batch of 12 designs of 16x8x8 to 50x25x25 elements took 63 ms here and 77 to 87 ms in
 // one persistent kernel with the CTAs shared out: a system there has too few CTAs for a march, whose
 // steps follow one another, and all wait for the slowest between launches.
 //
@@ -1341,6 +1341,26 @@ static void vecset_free(VecSet &v) {
     v = VecSet();
 }
 
+// Whether an iteration of this system, whose matrices have the modal form, is sooner in that form than on the tensor
+// cores, beside m - 1 other systems there.  The march rounds a grid up to its tiles and to rounds of one per SM
+// (65^3 fills 61% of the columns it takes, 128x64x64 all), the bricks of 8x4x4 hardly.  Times in us by fits to 185 single
+// solves of 2.5e4 to 2.2e6 elements, both forms measured (modal and tensor cores: 76.3 and 67.6 at 65^3, 118 and 107 at
+// 132x66x66, 39.7 and 36.2 at 33x52x49, 70 and 97 at 128x64x64, 45 and 58 at 93x54x47): by the slower one 14 of the 185
+// lost up to 11%, by this rule 9 lose 1 to 5%.  A batch shares the 21 us that two launches and the vector step's barrier
+// take; together and by itself then, two systems, us an iteration: 52.6 and 66.4 at 104x52x52, 59 and 77 at 65^3, 89 and
+// 70 at 128x64x64.  The vector step takes a row of control points in passes of a warp, which show where rows are few and
+// long (1000x17x17: 129 and 77).
+static bool modal_sooner(const Op &op, size_t m) {
+    const ModalTile &t = op.mixed->mt;
+    const double c = t.clocks / 1965.0;
+    const double modal = t.nt == 0 ? 10.8 + 1.1 * c : (t.nt <= 256 ? 5.6 + 1.52 * c : 1.1 + 1.6 * c);
+    const Geom &g = op.g;
+    const int passes = (g.cx + 31) / 32;
+    const bool few = (long long)g.cy * g.cz < (long long)op.num_sms * 4 * (kTailThreads / 32);
+    const double tc = 21.0 / (double)m + 2.77 * g.nbricks / op.num_sms + (few && passes > 5 ? 1.6 * (passes - 5) : 0.0);
+    return modal <= tc;
+}
+
 // CTAs of the fused vector step that can be resident at once (its grid barrier needs all of them)
 static int tail_capacity(const Op &op) { return op.mixed->tail_per_sm * op.num_sms; }
 
@@ -2042,6 +2062,8 @@ int mixed_solve(Op &op, const double *b, const double *diag, double tol, int64_t
     if (rc) return rc;
     if ((rc = mixed_init(op))) return rc;
     MixedState &ms = *op.mixed;
+    const bool modal = op.modal.ok && modal_sooner(op, 1);
+    if (!modal && ((rc = mixed_init_tc(op)) || (rc = vecset_tc(op, ms.v)))) return rc;
     const int check_every = opts.check_every > 0 ? opts.check_every : 32;
     std::vector<MixedItem> items(1);
     items[0].op = &op;
@@ -2069,7 +2091,7 @@ int mixed_solve(Op &op, const double *b, const double *diag, double tol, int64_t
     bt.bmat = ms.d_bmat;
     bt.limit = op.grid_wait_limit;
     bt.graph = ms.graph;
-    if (op.modal.ok) {
+    if (modal) {
         if ((rc = set_modal(bt, op, ms.v))) return rc;
     } else if (!ms.graph || ms.graph_batch != check_every || ms.graph_limit != op.grid_wait_limit) {
         const TcInst I = make_inst(op, ms.v, ms.d_state, 0, bt.tail_grid, 1.f);
@@ -2212,11 +2234,10 @@ static int autotune(MixedBatch &bt, std::vector<MixedItem> &items, int max_per_s
     return rc;
 }
 
-// Elements from which the systems of a batch are solved one after another on the modal kernel instead of
-// together on the tensor-core kernels: such a system fills the chip by itself, and its iterations are shorter
-// (70 us against 97 at 128x64x64).  Measured, together and one after another: 4 systems of 80x40x40 143 and 161 ms, of
-// 96x48x48 210 and 204 ms, of 128x64x64 660 and 485 ms.
+// Elements from which a system of a batch may leave it and be solved by itself (solve_alone): a smaller one does not
+// fill the chip.
 constexpr long long kSoloElements = 1LL << 18;
+static bool solve_alone(const Op &op, size_t m) { return op.nel >= kSoloElements && modal_sooner(op, m); }
 
 // Several systems at once: systems m of the call are (ops[m], vsets[m]) with right-hand side b[m]
 // (device), Jacobi diagonal diag[m] (device, null: the operator's own), tolerance tol[m] and
@@ -2283,7 +2304,7 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
     if ((int)m > cap || (int)m > kMaxInst)
         return set_error(ICC_BAD_ARG, "batched mixed solve: more systems than resident CTAs of the vector step");
     if (modal && m > 1) {
-        // systems that fill the chip go one after another on the modal kernel, the others together
+        // systems that fill the chip and are sooner there go one after another on the modal kernel, the others together
         std::vector<size_t> together;
         auto part = [&](const std::vector<size_t> &idx) {
             std::vector<Op *> o;
@@ -2314,12 +2335,14 @@ int mixed_solve_batch(cudaStream_t stream, const std::vector<Op *> &ops, const s
             return (int)ICC_OK;
         };
         for (size_t i = 0; i < m; ++i)
-            if (ops[i]->nel < kSoloElements) together.push_back(i);
+            if (!solve_alone(*ops[i], m)) together.push_back(i);
         if (together.size() < m) {
             for (size_t i = 0; i < m; ++i)
-                if (ops[i]->nel >= kSoloElements && (rc = part({i}))) return rc;
+                if (solve_alone(*ops[i], m) && (rc = part({i}))) return rc;
             return together.empty() ? ICC_OK : part(together);
         }
+    }
+    if (modal && (m > 1 || !modal_sooner(*ops[0], 1))) {
         modal = false;
         for (size_t i = 0; i < m; ++i)
             if ((rc = mixed_init_tc(*ops[i])) || (rc = vecset_tc(*ops[i], *vsets[i]))) return rc;

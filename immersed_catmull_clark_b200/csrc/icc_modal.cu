@@ -197,6 +197,7 @@ static void modal_plan(const Geom &g, int sms, ModalTile &best) {
     double cost = std::fmax(f64 ? 7500.0 : 6700.0, (double)cubes.n / sms * (f64 ? 7000.0 : 4800.0));
     best.nt = 0;
     best.t = cubes;
+    best.clocks = cost;
     // clocks of an element step and of a plane-only step by columns
     struct Step { int nt; double el, pl; };
     const Step f64_steps[] = {{128, 5400.0, 2400.0}, {256, 7000.0, 3100.0}};
@@ -216,7 +217,7 @@ static void modal_plan(const Geom &g, int sms, ModalTile &best) {
                     if (n > 1e9) break;
                     const double c = std::ceil(n / sms) * (tz * st[q].el + 5 * st[q].pl);
                     if (c < cost) {
-                        cost = c;
+                        cost = best.clocks = c;
                         best.nt = st[q].nt;
                         best.t = make_tiles(g.nx, g.ny, g.nz, tx, ty, tz);
                     }

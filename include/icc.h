@@ -170,7 +170,7 @@ int icc_apply_f64_noalloc(const int64_t nel_dir[3], const double *ke_types_dev, 
 /* Many independent solves (designs of uneven sizes, or load cases) at once: instance i solves
  * ops[i] x[i] = b[i] as icc_pcg_solve does (diag may be NULL, or diag[i] NULL), all instances in
  * flight together on their handles' streams (ICC_MIXED: instances of 2^18 or more elements one
- * after another, the others in one batch).  Per instance: status[i] (an icc_pcg_solve code),
+ * after another where that is sooner, the others in one batch).  Per instance: status[i] (an icc_pcg_solve code),
  * iters[i], rel_res[i] (both may be NULL).  Returns ICC_OK when every instance ran (converged or
  * not), else the first instance's error.  The handles must be distinct. */
 int icc_pcg_solve_batched(int32_t count, icc_op *const *ops, const double *const *b, const double *const *diag,
@@ -208,7 +208,8 @@ void icc_topopt_destroy(icc_topopt *t);
 /* Several load cases (extends the reference's single tip load, which the handle starts with):
  * forces is nload x ndof (component-blocked, like every vector here).  Each design iteration then
  * solves every case warm-started from its previous state.  With cfg.precision = ICC_MIXED and
- * nload > 1 the cases' state solves run as one batch (from 2^18 elements on one after another):
+ * nload > 1 the cases' state solves run as one batch (from 2^18 elements on one after another
+ * where that is sooner):
  * every PCG iteration is one tensor-core apply over the bricks of all cases and one fused vector
  * step (per-case PCG scalars, each case stops on its own tolerance).  With ICC_FP64 the cases are solved one after another.
  * Compliance and element energies are summed over the cases, and pcg_iters reports the sum. */
