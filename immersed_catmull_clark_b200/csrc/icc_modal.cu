@@ -165,12 +165,12 @@ bool modal_setup(const Op &op, ModalHost &m) {
             congruence(R[0], R[1], R[2], ku.data(), kt.data());
             const double *K = op.host_ktypes.data() + (size_t)t * 81 * 81;
             double kmax = 0.0;   // the squares below must neither overflow nor vanish
-            for (int i = 0; i < 81 * 81; ++i) kmax = std::fmax(kmax, std::fabs(K[i]));
-            if (kmax == 0.0) kmax = 1.0;
+            for (int i = 0; i < 81 * 81; ++i) kmax = std::fabs(K[i]) > kmax ? std::fabs(K[i]) : kmax;
+            const double unit = kmax > 0.0 ? 1.0 / kmax : 1.0;
             double dev[81] = {}, norm[81] = {};
             for (int i = 0; i < 81; ++i)
                 for (int j = 0; j < 81; ++j) {
-                    const double k = K[i * 81 + j] / kmax, d = kt[(size_t)i * 81 + j] / kmax - k;
+                    const double k = K[i * 81 + j] * unit, d = kt[(size_t)i * 81 + j] * unit - k;
                     dev[j] += d * d;
                     norm[j] += k * k;
                 }
