@@ -1925,8 +1925,10 @@ static int set_modal(MixedBatch &bt, Op &op, VecSet &v) {
 static int run_mixed(MixedBatch &bt, std::vector<MixedItem> &items, const icc_solve_opts &opts, int64_t *launches_out) {
     cudaStream_t s = bt.stream;
     const size_t m = items.size();
-    // 0.6: a replacement every ~75 iterations at 128x64x64 keeps the FP32 recurrence close to the
-    // FP64 iteration count (1,350-1,410 vs 1,337 over four seeds; 0.1 gave up to 1,820)
+    // 0.6: a replacement every ~75 iterations at 128x64x64.  On the tensor cores 0.1 gave up to 1,820 iterations to 1e-8
+    // where 0.6 gave 1,350-1,410; the modal form does not depend on it between 0.3 and 0.9.  Iterations of six smoothed
+    // designs: FP64 1,334-1,344 to 1e-8 and 1,451-1,470 to 1e-10, modal form 1,339-1,436 and 1,794-2,014, tensor
+    // cores 1,432-1,808 and 1,997-2,159.
     const double delta = opts.inner_tol > 0.0 ? opts.inner_tol : 0.6;
     const int max_updates = opts.max_outer > 0 ? opts.max_outer : 1000;
     const int check_every = opts.check_every > 0 ? opts.check_every : 32;

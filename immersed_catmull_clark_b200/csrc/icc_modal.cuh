@@ -844,9 +844,10 @@ __device__ __forceinline__ void modal_others(const ModalSys<T> &S, const ModalNo
 // two (one barrier more: p'Ap needs the whole direction).  The loop ends when the state says so.
 //
 // One launch for many iterations instead of four (FP64) or two (FP32) per iteration, because at 24x16x12 an
-// iteration is two phases' and two barriers' latency (9,000 + 3,300 clocks and 2 x 4,000 of FP64) and the
-// launches between them came on top: FP64 46 -> 12.9 us, FP32 27 -> 12.5 us an iteration.  At 128x64x64 the march
-// bounds it: FP64 152,000 clocks and FP32 102,000 of an iteration (447 -> 105 us and 97 -> 70 us).  The march
+// iteration is a chain of latencies (FP64, 25,000 clocks: the apply 8,600, the vector step 3,100, two sums over a CTA,
+// two barriers and two totals of the CTAs' partials the rest) and the launches between them came on top: FP64 46 ->
+// 12.6 us, FP32 27 -> 12.4 us an iteration.  At 128x64x64 the march bounds it: FP64 156,000 of 215,000 clocks, FP32
+// 101,000 of 137,000 (447 -> 105 us and 97 -> 70 us).  The march
 // has one CTA per SM: its state fills the SM's tensor memory and its exchange most of the shared memory.
 template <class T, int NT>
 __host__ __device__ constexpr int modal_threads() { return NT == 0 ? 2 * kCubeThreads : ModalMarch<T>::max_nt; }

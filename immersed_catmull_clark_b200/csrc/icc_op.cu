@@ -1,7 +1,7 @@
 // Matrix-free p = 2 B-spline elasticity operator, Jacobi diagonal and device PCG for sm_100a.
 //
-// Work decomposition.  The element grid is cut into bricks of BX x BY x BZ = 8 x 4 x 4
-// elements.  One CTA owns one brick:
+// Isotropic element matrices take the kernels of icc_modal.cuh.  Work decomposition for all others:
+// the element grid is cut into bricks of BX x BY x BZ = 8 x 4 x 4 elements.  One CTA owns one brick:
 //   1. it stages the brick's (BX+2)(BY+2)(BZ+2) control-point patch of the input vector, all
 //      three components, into shared memory (input mask applied on the fly);
 //   2. its warps contract the gathered element vectors with the element matrices on the FP64

@@ -11,7 +11,7 @@ belongs to the lower rank) and are summed over ranks with one all-reduce for p'A
 (r'r, r'z) per iteration; the recurrence, its stopping rule and its breakdown rule are those of
 rust/src/solver.rs:14-76.
 
-The mixed-precision form (SlabMixedPcg) runs the same recurrence in FP32 on the tensor-core apply
+The mixed-precision form (SlabMixedPcg) runs the same recurrence in FP32 on the FP32 apply
 of every slab, with the halo sum in FP32, every dot product in FP64, and FP64 residual
 replacement across the slabs, as the single-GPU mixed solve does.
 
@@ -185,7 +185,7 @@ class SlabPcg:
 
 class SlabMixedPcg(SlabPcg):
     """The mixed-precision form over x-slabs (reliable updates).  The FP32 recurrence x32, r32, p
-    uses `apply32` (FP32 tensors in and out: the slab's tensor-core apply) and the halo sum in FP32;
+    uses `apply32` (FP32 tensors in and out: the slab's FP32 apply) and the halo sum in FP32;
     every dot product is accumulated in FP64 and summed over the ranks.  Whenever the FP32 residual
     has fallen by `delta` since the last replacement, or after `seg` iterations, or when it meets
     the tolerance, the FP32 solution is added to the FP64 solution, the FP64 true residual
@@ -270,7 +270,7 @@ def device_apply(op):
 
 
 def device_apply_f32(op):
-    """The local FP32 apply of a slab's device operator on the tensor cores (FP32 torch tensors)."""
+    """The local FP32 apply of a slab's device operator (FP32 torch tensors)."""
     def apply(x):
         y = torch.empty_like(x)
         torch.cuda.current_stream().synchronize()
@@ -282,7 +282,7 @@ def device_apply_f32(op):
 
 def slab_operator(icc, slab, global_bounds, em_global, scale_global, free_mask_global, mask_mode, space=None):
     """The device operator of a slab: the slab's window of the global space (local numbering, the
-    global B-splines, so the operator also runs on the tensor cores next to a cut), the global
+    global B-splines, so the operator takes the same kernels next to a cut), the global
     element types restricted to the slab, the slab's element scales and mask.  `space` is the global
     SpaceBox (built from global_bounds and the slab's grid when not given)."""
     if space is None:
