@@ -298,19 +298,20 @@ cudaError_t launch_modal_apply(cudaStream_t s, const ModalHost &m, const ModalSy
 template cudaError_t launch_modal_apply<double>(cudaStream_t, const ModalHost &, const ModalSys<double> &, const ModalTile &);
 template cudaError_t launch_modal_apply<float>(cudaStream_t, const ModalHost &, const ModalSys<float> &, const ModalTile &);
 
-// Every CTA takes more than half of an SM's shared memory, so two of these kernels (two solves on two
-// streams) never share an SM: tensor memory is then always there for a resident CTA, and no CTA waits
-// for it while others wait for that CTA at a barrier.
+// Every CTA of a march takes more than half of an SM's shared memory, so two of these kernels (two solves on
+// two streams) never share an SM: tensor memory is then always there for a resident CTA, and no CTA waits
+// for it while others wait for that CTA at a barrier.  Cubes use no tensor memory.
 template <class T, int NT>
 static cudaError_t launch_pcg(cudaStream_t s, const ModalHost &m, const ModalSys<T> &S, const ModalTile &t, int iters, int *err,
                               long long limit) {
-    const int values = NT == 0 ? modal_threads<T, NT>() / kCubeThreads * kCubeSmem : march_smem(NT, t.t.ltx, true);
+    constexpr bool cube = NT <= kCubePair;
+    const size_t smem = (size_t)(cube ? NT * kCubeSmem : march_smem(NT, t.t.ltx, true)) * sizeof(T);
     cudaError_t e = cudaFuncSetAttribute(modal_pcg_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)S.ncta);
     cfg.blockDim = dim3(modal_threads<T, NT>());
-    cfg.dynamicSmemBytes = std::max((size_t)values * sizeof(T), (size_t)120 * 1024);
+    cfg.dynamicSmemBytes = cube ? smem : std::max(smem, (size_t)120 * 1024);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;   // the barriers need every CTA resident
@@ -323,7 +324,8 @@ static cudaError_t launch_pcg(cudaStream_t s, const ModalHost &m, const ModalSys
 template <class T>
 cudaError_t launch_modal_pcg(cudaStream_t s, const ModalHost &m, const ModalSys<T> &S, const ModalTile &t, int iters, int *err,
                              long long limit) {
-    if (t.nt == 0) return launch_pcg<T, 0>(s, m, S, t, iters, err, limit);
+    if (t.nt == 0)
+        return t.t.n <= S.ncta ? launch_pcg<T, kCubeOne>(s, m, S, t, iters, err, limit) : launch_pcg<T, kCubePair>(s, m, S, t, iters, err, limit);
     if (t.nt == 128) return launch_pcg<T, 128>(s, m, S, t, iters, err, limit);
     if (t.nt == 256) return launch_pcg<T, 256>(s, m, S, t, iters, err, limit);
     if constexpr (sizeof(T) == 4) return launch_pcg<T, 512>(s, m, S, t, iters, err, limit);

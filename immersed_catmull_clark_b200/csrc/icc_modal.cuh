@@ -844,18 +844,25 @@ __device__ __forceinline__ void modal_others(const ModalSys<T> &S, const ModalNo
 // two (one barrier more: p'Ap needs the whole direction).  The loop ends when the state says so.
 //
 // One launch for many iterations instead of four (FP64) or two (FP32) per iteration, because at 24x16x12 an
-// iteration is a chain of latencies (FP64, 25,000 clocks: the apply 8,600, the vector step 3,100, two sums over a CTA,
+// iteration is a chain of latencies (FP64, 24,000 clocks: the apply 10,100, the vector step 2,400, two sums over a CTA,
 // two barriers and two totals of the CTAs' partials the rest) and the launches between them came on top: FP64 46 ->
 // 12.6 us, FP32 27 -> 12.4 us an iteration.  At 128x64x64 the march bounds it: FP64 156,000 of 215,000 clocks, FP32
 // 101,000 of 137,000 (447 -> 105 us and 97 -> 70 us).  The march
 // has one CTA per SM: its state fills the SM's tensor memory and its exchange most of the shared memory.
+//
+// NT: columns of a march; kCubeOne or kCubePair for cubes, one or two at a time a CTA.  A system of no more cubes than
+// SMs takes CTAs of one, of which an SM holds two, so that such systems on several streams (a batch of FP64
+// solves, threads of the host) run beside one another: 16 FP64 designs of 24x12x12 to 32x16x16 in one call 80.8 -> 37.5
+// ms, a mixed solve of 24x16x12 with eight threads at it 3.43 -> 2.02 ms, by itself 8.2 as before.  Three FP32 CTAs
+// an SM spill (296 B; 16.0 us an iteration at 24x16x12 instead of 12.4).
+constexpr int kCubeOne = 1, kCubePair = 2;
 template <class T, int NT>
-__host__ __device__ constexpr int modal_threads() { return NT == 0 ? 2 * kCubeThreads : ModalMarch<T>::max_nt; }
+__host__ __device__ constexpr int modal_threads() { return NT <= kCubePair ? NT * kCubeThreads : ModalMarch<T>::max_nt; }
 
 template <class T, int NT>
-__global__ void __launch_bounds__((modal_threads<T, NT>()), 1)
+__global__ void __launch_bounds__((modal_threads<T, NT>()), NT == kCubeOne ? 2 : 1)
 modal_pcg_kernel(const __grid_constant__ ModalK<T> K, const __grid_constant__ ModalSys<T> S, int iters, int *err, long long limit) {
-    constexpr bool CUBE = NT == 0;
+    constexpr bool CUBE = NT <= kCubePair;
     constexpr int CT = modal_threads<T, NT>(), kGroups = CUBE ? CT / kCubeThreads : 1;
     extern __shared__ __align__(16) unsigned char modal_raw[];
     __shared__ uint32_t tmem_base;
