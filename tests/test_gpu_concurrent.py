@@ -43,3 +43,30 @@ def test_concurrent_solves_equal_single_ones(sizes, precision):
         t.join()
     for a, b in zip(single, out):
         assert b is not None and a[1] == b[1] and a[2] == b[2] and np.array_equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("precision", [icc.FP64, icc.MIXED])
+def test_applies_beside_a_solve(precision):
+    """Plain applies, whose marches take tensor memory as the solve's do, while another handle's solve runs."""
+    a, b, c = cantilever((64, 33, 40), 1), cantilever((70, 40, 30), 2), cantilever((33, 52, 49), 3)
+    x = [np.random.default_rng(i).standard_normal(s[0].ndof) for i, s in enumerate((b, c))]
+    ref = [(s[1].matvec(v), s[1].matvec_f32(v.astype(np.float32))) for s, v in zip((b, c), x)]
+    one = icc.PcgSolver(20000, 1e-7, precision=precision).solve(a[0].ndof, a[2], None, a[1])
+    out, done = [], threading.Event()
+
+    def solve():
+        for _ in range(3):
+            out.append(icc.PcgSolver(20000, 1e-7, precision=precision).solve(a[0].ndof, a[2], None, a[1]))
+        done.set()
+
+    t = threading.Thread(target=solve)
+    t.start()
+    same, n = True, 0
+    while not done.is_set() or n == 0:
+        for s, v, r in zip((b, c), x, ref):
+            same = same and np.array_equal(s[1].matvec(v), r[0]) and np.array_equal(s[1].matvec_f32(v.astype(np.float32)), r[1])
+        n += 1
+    t.join()
+    assert same and len(out) == 3
+    for o in out:
+        assert o[1] == one[1] and np.array_equal(o[0], one[0])
