@@ -51,7 +51,9 @@ typedef struct icc_op icc_op;
 
 typedef struct icc_solve_opts {
     int32_t precision;        /* ICC_FP64 or ICC_MIXED */
-    int32_t check_every;      /* PCG iterations between convergence checks on the host (0: 32) */
+    int32_t check_every;      /* PCG iterations between looks of the host at the solve's state, and between tests for a
+                                 residual replacement (0: 32); the device stops a solve by itself, so the form in
+                                 Legendre modes is looked at after up to eight of these */
     double inner_tol;         /* ICC_MIXED: the FP32 residual is replaced by the FP64 true residual
                                  whenever it has fallen by this factor since the last replacement
                                  (0: 0.6) */
